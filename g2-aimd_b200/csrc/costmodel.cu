@@ -41,44 +41,8 @@ static_assert(ModelView::N == G2_MODEL_PARAMS, "parameter layout");
 
 // ------------------------------------------------------------ features
 
-__device__ void root_features(const uint64_t *rp, const uint32_t *ci, const uint32_t *fo, const uint32_t *core,
-                              uint32_t v, float *f) {
-    const uint64_t lo = rp[v], hi = rp[v + 1];
-    const uint64_t s = lo + fo[v];
-    const uint32_t p = (uint32_t)(hi - s), nx = (uint32_t)(s - lo);
-    float wedge = 0.f, isum = 0.f, imax = 0.f;
-    for (uint32_t i = 0; i < p; i++) {
-        const uint32_t u = ci[s + i];
-        wedge += (float)(rp[u + 1] - rp[u] - fo[u]);
-    }
-    const uint32_t ns = p < 4 ? p : 4;
-    for (uint32_t j = 0; j < ns; j++) {
-        const uint32_t u = ci[s + (uint64_t)j * p / ns];
-        const uint64_t us = rp[u] + fo[u], ue = rp[u + 1];
-        uint32_t c = 0;
-        uint64_t pos = s;
-        for (uint64_t e = us; e < ue; e++) {  // |N+(u) ∩ N+(v)|, both sorted
-            const uint32_t y = ci[e];
-            pos = lower_bound(ci, pos, hi, y);
-            if (pos >= hi) break;
-            c += ci[pos] == y;
-        }
-        isum += (float)c;
-        imax = (float)c > imax ? (float)c : imax;
-    }
-    const float imean = ns ? isum / (float)ns : 0.f;
-    f[0] = log1pf((float)(hi - lo));
-    f[1] = log1pf((float)(core ? core[v] : p));
-    f[2] = log1pf((float)p);
-    f[3] = log1pf((float)nx);
-    f[4] = log1pf(wedge);
-    f[5] = log1pf(imean);
-    f[6] = p ? imean / (float)p : 0.f;
-    f[7] = log1pf(imax);
-}
-
 // One warp per root: lanes share the wedge sum and each sampled intersection
-// (integer sums, so the result equals root_features() exactly).
+// (integer sums).
 __global__ void features_kernel(const uint64_t *rp, const uint32_t *ci, const uint32_t *fo, const uint32_t *core,
                                 const uint32_t *src, uint64_t n, float *out) {
     const uint32_t lane = lane_id();
@@ -393,45 +357,76 @@ __global__ void adam_kernel(float *params, float *mom, float *vel, const float *
 
 // ------------------------------------------------------------- inference
 
-// Features + MLP of every root in one kernel (the inference fused into task
-// generation).  pred[i] (optional) = normalised log-cost of root src[i];
-// cost[i] (optional) = decoded cost (>= 1); *total (optional) += sum of costs.
-// With X given, the features are read from X instead: row src[i] (per-vertex
-// features cached for the loaded graph) or row i when src is null.
-__global__ void __launch_bounds__(128) score_kernel(const uint64_t *rp, const uint32_t *ci, const uint32_t *fo,
-                                                    const uint32_t *core, const uint32_t *src, uint64_t n,
-                                                    const float *X, const float *params, const float *norm,
-                                                    float *pred, float *cost, float *total) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    SharedModel &m = *reinterpret_cast<SharedModel *>(smem_raw);
-    WarpTile *tiles = reinterpret_cast<WarpTile *>(smem_raw + sizeof(SharedModel));
-    stage_model(m, params, norm);
-    const int w = threadIdx.x >> 5, lane = lane_id();
-    WarpTile &t = tiles[w];
-    const float ymean = norm[2 * F], ystd = norm[2 * F + 1];
-    float local = 0.f;
-    for (uint64_t base = ((uint64_t)blockIdx.x * 4 + w) * 16; base < n; base += (uint64_t)gridDim.x * 4 * 16) {
-        if (lane < 16) {
-            const uint64_t i = base + lane;
-            if (i < n) {
-                float f[F];
-                if (X) {  // precomputed features, rows indexed by vertex when src is given
-                    const uint64_t row = src ? (uint64_t)src[i] : i;
-                    for (int k = 0; k < F; k++) f[k] = X[row * F + k];
-                }
-                else
-                    root_features(rp, ci, fo, core, src ? src[i] : (uint32_t)i, f);
-                normalise_row(m, f, t.x[lane]);
-            } else {
-                for (int k = 0; k < KP; k++) t.x[lane][k] = 0.f;
-            }
+// MLP inference over feature rows (rows indexed by src when given), a warp per
+// 16 rows.  The weights stay in registers as bf16 B fragments and each layer's
+// accumulators are the next layer's A fragments (the C layout of two m16n8
+// tiles is the A layout of one m16k16), so nothing passes through shared
+// memory.  Bound by the feature rows' loads: 2^19 rows 249 us with weights and
+// activations staged in shared memory as fp32 and converted at every use.
+__global__ void __launch_bounds__(128) score_kernel(const uint32_t *src, uint64_t n, const float *X,
+                                                    const float *params, const float *norm, float *pred, float *cost,
+                                                    float *total) {
+    const int lane = lane_id(), g = lane >> 2, q = lane & 3;
+    uint32_t w1[H / 8], w2[H / 8][H / 16][2];  // layer 1 has 8 inputs: k >= 8 is zero
+    float2 b1[H / 8], b2[H / 8], w3[H / 8];
+#pragma unroll
+    for (int nt = 0; nt < H / 8; nt++) {
+        const float *r1 = params + ModelView::W1 + (nt * 8 + g) * F + 2 * q;
+        w1[nt] = pack_bf16(r1[0], r1[1]);
+#pragma unroll
+        for (int kt = 0; kt < H / 16; kt++) {
+            const float *r2 = params + ModelView::W2 + (nt * 8 + g) * H + kt * 16 + 2 * q;
+            w2[nt][kt][0] = pack_bf16(r2[0], r2[1]);
+            w2[nt][kt][1] = pack_bf16(r2[8], r2[9]);
         }
-        __syncwarp();
-        forward16(m, t);
-        if (lane < 16) {
-            const uint64_t i = base + lane;
+        const int col = nt * 8 + 2 * q;
+        b1[nt] = make_float2(params[ModelView::B1 + col], params[ModelView::B1 + col + 1]);
+        b2[nt] = make_float2(params[ModelView::B2 + col], params[ModelView::B2 + col + 1]);
+        w3[nt] = make_float2(bf16r(params[ModelView::W3 + col]), bf16r(params[ModelView::W3 + col + 1]));
+    }
+    const float b3 = params[ModelView::B3];
+    const float m0 = norm[2 * q], m1 = norm[2 * q + 1], s0 = 1.f / norm[F + 2 * q], s1 = 1.f / norm[F + 2 * q + 1];
+    const float ymean = norm[2 * F], ystd = norm[2 * F + 1];
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    float local = 0.f;
+    auto row_of = [&](uint64_t i) { return i < n ? (src ? (uint64_t)src[i] : i) : ~0ull; };
+    auto load = [&](uint64_t row) {
+        if (row == ~0ull) return make_float2(0.f, 0.f);
+        const float *f = X + row * F + 2 * q;
+        return make_float2((f[0] - m0) * s0, (f[1] - m1) * s1);
+    };
+    for (uint64_t base = warp * 16; base < n; base += nwarps * 16) {
+        const float2 x0 = load(row_of(base + g)), x1 = load(row_of(base + g + 8));
+        const uint32_t ax[4] = {pack_bf16(x0.x, x0.y), pack_bf16(x1.x, x1.y), 0u, 0u};
+        uint32_t h[H / 16][4];
+#pragma unroll
+        for (int nt = 0; nt < H / 8; nt++) {
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+            const uint32_t b[2] = {w1[nt], 0u};
+            mma16816(c, ax, b);
+            const int kt = nt >> 1, hi = (nt & 1) * 2;
+            h[kt][hi] = pack_bf16(fmaxf(c[0] + b1[nt].x, 0.f), fmaxf(c[1] + b1[nt].y, 0.f));
+            h[kt][hi + 1] = pack_bf16(fmaxf(c[2] + b1[nt].x, 0.f), fmaxf(c[3] + b1[nt].y, 0.f));
+        }
+        float y0 = 0.f, y1 = 0.f;  // rows g and g + 8, this lane's columns
+#pragma unroll
+        for (int nt = 0; nt < H / 8; nt++) {
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int kt = 0; kt < H / 16; kt++) mma16816(c, h[kt], w2[nt][kt]);
+            y0 += bf16r(fmaxf(c[0] + b2[nt].x, 0.f)) * w3[nt].x + bf16r(fmaxf(c[1] + b2[nt].y, 0.f)) * w3[nt].y;
+            y1 += bf16r(fmaxf(c[2] + b2[nt].x, 0.f)) * w3[nt].x + bf16r(fmaxf(c[3] + b2[nt].y, 0.f)) * w3[nt].y;
+        }
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            y0 += __shfl_xor_sync(G2_FULL, y0, o);
+            y1 += __shfl_xor_sync(G2_FULL, y1, o);
+        }
+        if (q < 2) {  // lane q = 0 writes row g, q = 1 row g + 8
+            const uint64_t i = base + g + 8 * q;
             if (i < n) {
-                const float y = t.y[lane];
+                const float y = (q ? y1 : y0) + b3;
                 const float c = expm1f(fminf(y * ystd + ymean, 80.f));  // targets are log1p(cycles)
                 const float cc = c > 1.f ? c : 1.f;
                 if (pred) pred[i] = y;
@@ -439,10 +434,9 @@ __global__ void __launch_bounds__(128) score_kernel(const uint64_t *rp, const ui
                 local += cc;
             }
         }
-        __syncwarp();
     }
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(G2_FULL, local, o);
-    if (lane == 0 && total) atomicAdd(total, local);
+    if (lane == 0 && total && local != 0.f) atomicAdd(total, local);
 }
 
 }  // namespace
@@ -471,12 +465,11 @@ cudaError_t adam_launch(float *params, float *mom, float *vel, const float *grad
     return cudaGetLastError();
 }
 
-cudaError_t score_launch(const uint64_t *rp, const uint32_t *ci, const uint32_t *fo, const uint32_t *core,
-                         const uint32_t *src, uint64_t n, const float *X, const float *params, const float *norm,
+cudaError_t score_launch(const uint32_t *src, uint64_t n, const float *X, const float *params, const float *norm,
                          float *pred, float *cost, float *total, int sms, cudaStream_t st) {
-    const size_t sm = model_smem_bytes();
-    cudaFuncSetAttribute(score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    score_kernel<<<sms * 4, 128, sm, st>>>(rp, ci, fo, core, src, n, X, params, norm, pred, cost, total);
+    const uint64_t blocks = (n + 63) / 64, cap = 4ull * (uint64_t)sms;
+    score_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks < cap ? blocks : cap), 128, 0, st>>>(src, n, X, params, norm,
+                                                                                         pred, cost, total);
     return cudaGetLastError();
 }
 

@@ -175,8 +175,7 @@ cudaError_t train_step_launch(const float *X, const float *Y, const uint32_t *id
                               const float *norm, float *grad, float *loss, cudaStream_t st);
 cudaError_t adam_launch(float *params, float *mom, float *vel, const float *grad, float lr, int step,
                         cudaStream_t st);
-cudaError_t score_launch(const uint64_t *rp, const uint32_t *ci, const uint32_t *fo, const uint32_t *core,
-                         const uint32_t *src, uint64_t n, const float *X, const float *params, const float *norm,
+cudaError_t score_launch(const uint32_t *src, uint64_t n, const float *X, const float *params, const float *norm,
                          float *pred, float *cost, float *total, int sms, cudaStream_t st);
 
 }  // namespace g2
