@@ -24,6 +24,25 @@ constexpr uint32_t kRecordBit = 0x80000000u;
 // Depth word of a record slot whose reservation ran past the buffer's end.
 constexpr uint32_t kVoidRecord = 0xffffffffu;
 
+// Bit rows of the last ids of a graph (g2_corebits.cuh): row of vertex u in
+// [base, end) = bits of N+(u) over the ids base, base + 1, ..., `stride` words
+// (a multiple of 4) each, from word `off` of the matrix.  A batch of graphs has
+// one block per graph; row0 = rows of the blocks before it.
+struct CoreBlock {
+    uint32_t base, end, stride, row0;
+    uint64_t off;
+};
+struct CoreBits {
+    const uint32_t *bits;
+    const CoreBlock *blocks;  // device; used if nblocks > 1
+    uint32_t nblocks, rows;   // rows = sum of the blocks' rows
+    CoreBlock one;            // the block if there is only one
+};
+// Block geometry of a graph of n vertices and m entries whose ids [lo, lo + n)
+// get bit rows on the last K, K^2 bits at most about `bytes` (K a multiple of 128
+// unless K = n); row0 / off continue from the previous block.
+CoreBlock core_block_of(uint32_t lo, uint32_t n, uint64_t bytes, uint32_t row0, uint64_t off);
+
 struct MceArgs {
     const uint64_t *rp;
     const uint32_t *ci;
@@ -153,6 +172,46 @@ uint32_t match_p0_words(int wpl, bool clique_path, uint32_t k, bool metrics);
 size_t match_smem_bytes(int wpl, int warps_per_block, uint32_t p0_words);
 cudaError_t match_launch(const DevPlan &plan, const MatchArgs &a, int blocks, int warps_per_block,
                          cudaStream_t st, bool clique_path, int wpl, int ctas_per_sm);
+
+// Counting of 3-, 4- and 5-cliques on core bit rows (clique.cu).
+struct CliqueArgs {
+    const uint64_t *rp;
+    const uint32_t *ci;
+    const uint32_t *fo;
+    const uint32_t *tasks;
+    const uint32_t *task_part;      // optional per task: (nparts << 16) | part of a split root
+    uint64_t ntasks;
+    const unsigned long long *ntasks_dev;  // optional: task count read from device memory
+    CoreBits core;
+    uint32_t *bits_out;             // the matrix, written by the preparation kernel
+    uint32_t in_order;              // one list in task order (else lists by root size)
+    uint32_t cta_min;               // lists by size: roots with larger |P0| are shared by a CTA
+    uint32_t p_fit;                 // roots with larger |P0| go to the rest list
+    uint32_t *lists;                // four lists of list_cap task ids: by size (or [0] in order), [3] rest
+    uint32_t *pieces;               // 5-cliques, lists by size: (pieces << 16) | piece of list 0's entries
+    uint64_t list_cap, extra_cap;   // list_cap >= ntasks + extra_cap; extra_cap = pieces beyond one per root
+    unsigned long long *counts;     // list lengths; [4] extra pieces
+    unsigned long long *heads;      // list heads
+    uint32_t chunk;                 // in-order runs: tasks per queue atomic
+    uint32_t *scratch;              // per-warp slabs
+    uint64_t words_per_warp;
+    uint32_t smem_words;            // dynamic shared memory of a CTA
+    uint32_t q_words;               // words of a candidate-set row (5-cliques), else 0
+    unsigned long long *out;
+    uint64_t *root_nodes;           // optional: embeddings counted per task
+    uint64_t *root_cost;            // optional: SM cycles per task
+    int *status;
+    const unsigned long long *deadline;
+};
+// Largest |P0| that one warp walks in runs by size.
+uint32_t clique_cta_min(uint32_t k);
+// Largest |P0| a launch of this geometry counts itself.
+uint32_t clique_p_fit(uint32_t k, bool in_order, uint64_t words_per_warp, int warps_per_block, uint32_t smem_words);
+// Dynamic shared memory (words) for roots up to max_fwd, and a row's word count for 5-cliques.
+uint32_t clique_smem_words(uint32_t k, bool in_order, uint32_t max_fwd, int warps_per_block, uint32_t *q_words);
+int clique_blocks_per_sm(uint32_t k, bool in_order, int warps_per_block, uint32_t smem_words);
+cudaError_t clique_prepare_launch(const CliqueArgs &a, uint32_t k, int sms, cudaStream_t st);
+cudaError_t clique_launch(const CliqueArgs &a, uint32_t k, int blocks, int warps_per_block, cudaStream_t st);
 
 // Sort each row of `in` (device CSR rows given by rp) into `out`, in calls of at
 // most max_chunk entries (kcore.cu); synchronous.

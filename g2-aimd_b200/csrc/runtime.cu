@@ -221,6 +221,13 @@ int sort_keys(g2_ctx *ctx, uint64_t n, bool estimates, cudaStream_t st) {
     return G2_OK;
 }
 
+// Does a run count its plan on core bit rows (clique.cu)?  3-, 4- and 5-cliques
+// unless the generic path or the work model is asked for.
+bool clique_run(const g2_ctx *ctx, const g2_opts *o) {
+    return ctx->clique_plan && ctx->plan.k >= 3 && ctx->plan.k <= 5 && !(o && o->intersect_mode == 1) &&
+           !(o && (o->flags & G2_FLAG_WORK_MODEL));
+}
+
 // Task generation: upload the roots, compute the schedule's cost per root (the
 // learned model's features + MLP run here, in one kernel), optionally split
 // heavy roots, sort the tasks by descending cost.  No host synchronisation.
@@ -236,11 +243,12 @@ int prepare_tasks(g2_ctx *ctx, const uint32_t *sources, uint64_t nsrc, bool on_d
     if (sched > G2_SCHED_LEARNED) return G2_ERR_INVALID;
     if (sched == G2_SCHED_SCORES && !(o && o->scores)) return G2_ERR_INVALID;
     if (sched == G2_SCHED_LEARNED && !ctx->d_model) return G2_ERR_INVALID;
-    // MCE balances inside roots by handing branches to idle warps, which split
+    // MCE balances inside roots by handing branches to idle warps, and 3- to
+    // 5-clique runs by sharing a root's rows among a CTA's warps, which split
     // tasks cannot do: there the static split is only taken when asked for
     const bool split = nsrc > 0 && (sched == G2_SCHED_HEURISTIC || sched == G2_SCHED_LEARNED) &&
-                       ((flags & G2_FLAG_SPLIT) ||
-                        (!mce && sched == G2_SCHED_LEARNED && !(flags & G2_FLAG_NO_SPLIT)));
+                       ((flags & G2_FLAG_SPLIT) || (!mce && !clique_run(ctx, o) && sched == G2_SCHED_LEARNED &&
+                                                    !(flags & G2_FLAG_NO_SPLIT)));
     // sum_i ceil(c_i / t) <= n + total / t = n + g * warps
     const uint32_t gran = (o && o->split_granularity) ? std::min<uint32_t>(o->split_granularity, 1024u) : 4u;
     const uint64_t cap = split ? nsrc + (uint64_t)gran * nwarps + 64 : nsrc;
@@ -359,6 +367,7 @@ int ensure_scratch(g2_ctx *ctx) {
 // Device counters: queue heads of the passes, deferred-list sizes, hand-off
 // record / pool allocation and the record queue.
 constexpr int kCtrHead = 0;    // 3 queue heads
+constexpr int kCtrClique = 4;  // clique runs: 4 list lengths, extra pieces, then 3 list heads
 constexpr int kCtrDefer = 16;  // 3 deferred-list sizes
 constexpr int kCtrRec = 19;    // records reserved
 constexpr int kCtrPool = 20;   // pool units (64 words) used
@@ -481,6 +490,51 @@ int gather_root_outputs(g2_ctx *ctx, const uint32_t *sources, uint64_t nsrc, uin
         }
     }
     return G2_OK;
+}
+
+// Matrix bytes of a graph's core: the bytes of its column array (K = 5.7 sqrt(m)
+// ids), at most 2 GiB.  4-cliques of R-MAT s20 / triangles of s18 in ms by bytes
+// per entry: 0.25 9.2 / 0.74, 1 7.0 / 0.49, 2 6.1 / 0.37, 4 6.1 / 0.34,
+// 16 6.2 / 0.33 (an earlier build of the kernels).
+uint64_t core_budget(uint64_t m) { return std::min<uint64_t>(std::max<uint64_t>(4 * m, 1u << 20), 2ull << 30); }
+
+// Geometry of the loaded graph's core bit rows; words = the matrix's size.
+g2::CoreBits core_geometry(const g2_ctx *ctx, uint64_t *words) {
+    g2::CoreBits cb{};
+    if (ctx->batch_off.size() > 2) {
+        cb.blocks = ctx->d_core_blocks;
+        cb.nblocks = (uint32_t)ctx->batch_off.size() - 1;
+        cb.rows = ctx->core_rows;
+        *words = ctx->core_words;
+    } else {
+        cb.nblocks = 1;
+        cb.one = g2::core_block_of(0, (uint32_t)ctx->n, core_budget(ctx->m), 0, 0);
+        cb.rows = cb.one.end - cb.one.base;
+        *words = (uint64_t)cb.rows * cb.one.stride;
+    }
+    return cb;
+}
+
+constexpr uint64_t kCliquePieces = 1u << 16;  // list entries for pieces of heavy roots
+
+// The core matrix and the task lists of clique runs over up to `tasks` tasks (0: the matrix alone):
+// G2_OK, or G2_ERR_OOM where the run has to do without them (no memory left, or
+// a stream capture, in which nothing is allocated).
+int ensure_clique(g2_ctx *ctx, uint64_t tasks, cudaStream_t st, g2::CoreBits *cb) {
+    uint64_t words = 0;
+    *cb = core_geometry(ctx, &words);
+    words = std::max<uint64_t>(words, 4);
+    if (tasks) tasks = 5 * (tasks + kCliquePieces);  // four lists and the pieces
+    if (ctx->core_bits_cap < words || ctx->clists_cap < tasks) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        G2_TRY(cudaStreamIsCapturing(st, &cs));
+        if (cs != cudaStreamCaptureStatusNone) return G2_ERR_OOM;
+    }
+    int rc = grow(ctx, ctx->d_core_bits, ctx->core_bits_cap, words, "core bit rows");
+    if (!rc && tasks) rc = grow(ctx, ctx->d_clists, ctx->clists_cap, tasks, "clique task lists");
+    if (rc == G2_ERR_OOM) cudaGetLastError();
+    cb->bits = ctx->d_core_bits;
+    return rc;
 }
 
 // Optional L2 persistence window over the tail of the column array (the dense
@@ -742,6 +796,28 @@ void match_geometry(g2_ctx *ctx, const g2_opts *o, int *wpl, int *wpb, int *bloc
 
 }  // namespace
 
+namespace {
+
+// Geometry of a clique run: CTA size, shared memory and grid.
+struct CliqueGrid {
+    bool in_order;
+    int wpb, blocks;
+    uint32_t smem_words, q_words;
+};
+CliqueGrid clique_grid(g2_ctx *ctx, const g2_opts *o) {
+    CliqueGrid g;
+    g.in_order = !o || o->schedule == G2_SCHED_GIVEN;
+    // a root shared by a CTA keeps 8 warps busy; its rows' shared memory bounds the
+    // CTAs per SM, so fewer warps per CTA would be fewer per SM
+    g.wpb = g.in_order ? default_warps(o) : 8;
+    g.smem_words = g2::clique_smem_words(ctx->plan.k, g.in_order, ctx->max_fwd, g.wpb, &g.q_words);
+    g.blocks = default_blocks(ctx, o, g.wpb,
+                              g2::clique_blocks_per_sm(ctx->plan.k, g.in_order, g.wpb, g.smem_words));
+    return g;
+}
+
+}  // namespace
+
 namespace g2rt {
 
 int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned long long *d_out,
@@ -803,12 +879,63 @@ int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned lo
         a.wait_cycles = (o && o->wait_cycles) ? o->wait_cycles : kWaitCycles;
         a.spill_cycles = 1000ull * ((o && o->spill_kcycles) ? o->spill_kcycles : kSpillKcycles);
     }
+    g2::CliqueArgs q{};
+    CliqueGrid cg{};
+    bool rows = clique_run(ctx, o);
+    if (rows) {
+        rc = ensure_clique(ctx, std::max<uint64_t>(tl.cap, 1), st, &q.core);
+        if (rc && rc != G2_ERR_OOM) return rc;
+        rows = rc == G2_OK;
+    }
+    if (rows) {
+        cg = clique_grid(ctx, o);
+        q.rp = ctx->d_rp;
+        q.ci = ctx->d_ci;
+        q.fo = ctx->d_fo;
+        q.tasks = ctx->d_tasks;
+        q.task_part = a.task_part;
+        q.ntasks = tl.cap;
+        q.ntasks_dev = a.ntasks_dev;
+        q.bits_out = ctx->d_core_bits;
+        q.in_order = cg.in_order;
+        q.lists = ctx->d_clists;
+        q.list_cap = ctx->clists_cap / 5;
+        q.extra_cap = kCliquePieces;
+        // a budgeted run drops an unfinished root whole: no pieces
+        if (ctx->plan.k == 5 && !a.deadline) q.pieces = ctx->d_clists + 4 * q.list_cap;
+        q.counts = ctx->d_ctr + kCtrClique;
+        q.heads = ctx->d_ctr + kCtrClique + 5;
+        q.chunk = std::min<uint32_t>((o && o->chunk) ? o->chunk : 1u, 32u);
+        q.scratch = ctx->d_scratch;
+        q.words_per_warp = (ctx->scratch_words / ((uint64_t)cg.blocks * cg.wpb)) & ~63ull;
+        q.smem_words = cg.smem_words;
+        q.q_words = cg.q_words;
+        q.cta_min = g2::clique_cta_min(ctx->plan.k);
+        q.p_fit = g2::clique_p_fit(ctx->plan.k, cg.in_order, q.words_per_warp, cg.wpb, cg.smem_words);
+        q.out = d_out;
+        q.root_nodes = d_root_nodes;
+        q.root_cost = d_root_cost;
+        q.status = ctx->d_status;
+        q.deadline = a.deadline;
+    }
     if (ctx->timed) G2_TRY(cudaEventRecord(ctx->ev[0], st));
     L2Window l2(ctx, st, flags);
-    cudaError_t e = g2::match_launch(ctx->plan, a, blocks, wpb, st, clique, wpl, o ? (int)o->ctas_per_sm : 0);
+    cudaError_t e = cudaSuccess;
+    if (rows) {
+        e = g2::clique_prepare_launch(q, ctx->plan.k, ctx->sm_count, st);
+        if (e == cudaSuccess) e = g2::clique_launch(q, ctx->plan.k, cg.blocks, cg.wpb, st);
+        if (e != cudaSuccess) return fail_cuda(ctx, e, "clique_launch");
+        ctx->launches += 2;
+        // roots wider than the rows' room, counted by the general kernel
+        a.task_index = q.lists + 3 * q.list_cap;
+        a.ntasks_dev = q.counts + 3;
+    }
+    if (!rows || ctx->max_fwd > q.p_fit) {
+        e = g2::match_launch(ctx->plan, a, blocks, wpb, st, clique, wpl, o ? (int)o->ctas_per_sm : 0);
+        ctx->launches++;
+    }
     if (e != cudaSuccess) return fail_cuda(ctx, e, "match_launch");
     if (ctx->timed) G2_TRY(cudaEventRecord(ctx->ev[1], st));
-    ctx->launches++;
     if (ctx->timed) ctx->timed_passes = 1;
     return G2_OK;
 }
@@ -914,6 +1041,9 @@ int g2_reserve(g2_ctx *ctx, uint64_t max_sources) {
         if (!rc) rc = grow(ctx, ctx->d_xparts, ctx->xparts_cap, cap, "expanded parts");
         if (!rc && !ctx->d_ntask) rc = grow(ctx, ctx->d_ntask, ctx->ntask_cap, 1, "task count");
         if (rc) return rc;
+        g2::CoreBits cb;
+        rc = ensure_clique(ctx, ctx->tasks_cap, nullptr, &cb);
+        if (rc && rc != G2_ERR_OOM) return rc;
         size_t sort_need = 0, scan_need = 0;
         cub::DeviceRadixSort::SortKeys(nullptr, sort_need, ctx->d_keys, ctx->d_keys2, (int)cap, 0, 64);
         cub::DeviceScan::ExclusiveSum(nullptr, scan_need, ctx->d_S, ctx->d_S, (int)max_sources);
@@ -1065,7 +1195,7 @@ int g2_close(g2_ctx *ctx) {
                     ctx->d_roots,  ctx->d_S,       ctx->d_part,    ctx->d_xroots, ctx->d_xparts,     ctx->d_cost,
                     ctx->d_total,  ctx->d_ntask,   ctx->d_cub,     ctx->d_model,  ctx->d_work,
                     ctx->d_feat,   ctx->d_rec,     ctx->d_pool,    ctx->d_ready,  ctx->d_goff,    ctx->d_fwdmax,
-                    ctx->d_epoch,  ctx->d_deadline,
+                    ctx->d_epoch,  ctx->d_deadline, ctx->d_core_bits, ctx->d_clists, ctx->d_core_blocks,
                     ctx->d_root_cliques, ctx->d_gcount};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -1355,6 +1485,23 @@ int g2_batch_load(g2_ctx *ctx, const g2_batch_graph *graphs, uint32_t ngraphs) {
     if (!rc) rc = grow(ctx, ctx->d_goff, ctx->goff_cap, ngraphs + 1, "batch offsets");
     if (rc) return rc;
     G2_TRY(cudaMemcpy(ctx->d_goff, off.data(), sizeof(uint64_t) * (ngraphs + 1), cudaMemcpyHostToDevice));
+    // core bit rows of each graph, the batch's matrix budget dealt out by entries
+    std::vector<g2::CoreBlock> blocks(ngraphs);
+    ctx->core_rows = 0;
+    ctx->core_words = 0;
+    const uint64_t budget = core_budget(m);
+    for (uint32_t g = 0; g < ngraphs; g++) {
+        const double share = m ? (double)graphs[g].m / (double)m : 0.0;
+        blocks[g] = g2::core_block_of((uint32_t)off[g], (uint32_t)graphs[g].n, (uint64_t)(share * (double)budget),
+                                      ctx->core_rows, ctx->core_words);
+        const uint32_t rows = blocks[g].end - blocks[g].base;
+        ctx->core_rows += rows;
+        ctx->core_words += (uint64_t)rows * blocks[g].stride;
+    }
+    rc = grow(ctx, ctx->d_core_blocks, ctx->core_blocks_cap, std::max<uint32_t>(ngraphs, 1u), "core blocks");
+    if (rc) return rc;
+    if (ngraphs)
+        G2_TRY(cudaMemcpy(ctx->d_core_blocks, blocks.data(), sizeof(g2::CoreBlock) * ngraphs, cudaMemcpyHostToDevice));
     ctx->batch_off = off;
     return G2_OK;
 }

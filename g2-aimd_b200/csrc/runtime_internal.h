@@ -43,6 +43,14 @@ struct g2_ctx {
     uint32_t *d_ready = nullptr;          // their ready words
     uint32_t *d_epoch = nullptr;          // epoch of the current run (bumped on the device)
     uint32_t *d_pool = nullptr;           // MCE spill row pool
+    uint32_t *d_core_bits = nullptr;      // bit rows of the dense core (clique runs), rebuilt by every run
+    uint64_t core_bits_cap = 0;
+    uint32_t *d_clists = nullptr;         // clique runs: four lists of task ids
+    uint64_t clists_cap = 0;
+    g2::CoreBlock *d_core_blocks = nullptr;  // core blocks of a batch's graphs
+    uint64_t core_blocks_cap = 0;
+    uint32_t core_rows = 0;               // rows and words of the batch's core blocks
+    uint64_t core_words = 0;
     int *d_status = nullptr;
     unsigned long long *d_deadline = nullptr;  // %globaltimer ns of a run's time budget
     unsigned long long *d_out = nullptr;  // counters for the host entry points

@@ -100,15 +100,17 @@ typedef struct g2_plan {
 #define G2_SCHED_SCORES 2     /* descending caller scores                          */
 #define G2_SCHED_LEARNED 3    /* descending cost predicted on the device by the model
                                  set with g2_set_model (features + MLP fused into
-                                 task generation); GMatch splits heavy roots by
-                                 default                                          */
+                                 task generation); plan walks split heavy roots by
+                                 default (3- to 5-clique runs share them among a
+                                 CTA's warps instead)                             */
 
 /*
  * Run options.  Zero-initialise and set what you need; 0 means "default".
  */
 typedef struct g2_opts {
     uint32_t blocks;            /* persistent CTAs (default: 148 x occupancy)       */
-    uint32_t warps_per_block;   /* default 8                                        */
+    uint32_t warps_per_block;   /* default 8 (3- to 5-clique runs in schedule order
+                                   always use 8: a CTA shares its heavy roots)      */
     uint32_t schedule;          /* G2_SCHED_*                                       */
     uint32_t split_granularity; /* heavy-root splits aim at tasks of cost
                                    total / (granularity x warps) (0 = 4)           */
@@ -129,8 +131,8 @@ typedef struct g2_opts {
                                    many thousand SM cycles a walk checks for idle
                                    warps and hands them the pending work of its
                                    shallowest open level (0 = 20)                   */
-    uint32_t ctas_per_sm;       /* GMatch register budget, as CTAs of 256 threads per
-                                   SM: 0 or 4 (64 registers), 6 (40 registers, more
+    uint32_t ctas_per_sm;       /* GMatch register budget (not for 3- to 5-clique
+                                   runs), as CTAs of 256 threads per SM: 0 or 4 (64 registers), 6 (40 registers, more
                                    resident warps; pays on graphs larger than L2)   */
     uint32_t wait_cycles;       /* hang guard: the longest a warp waits for a handed-off
                                    record, in SM cycles (0 = 2^37, about 70 s); a run
