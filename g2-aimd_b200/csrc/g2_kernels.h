@@ -216,10 +216,10 @@ cudaError_t clique_launch(const CliqueArgs &a, uint32_t k, int blocks, int warps
 // Sort each row of `in` (device CSR rows given by rp) into `out`, in calls of at
 // most max_chunk entries (kcore.cu); synchronous.
 cudaError_t sort_rows_device(const uint64_t *rp, uint64_t n, uint64_t m, const uint32_t *in, uint32_t *out,
-                             uint64_t max_chunk, int sms);
+                             uint64_t max_chunk, int sms, uint64_t big_min = ~0ull);
 // Degeneracy order of a CSR on the device (kcore.cu); synchronous.
-cudaError_t degeneracy_order_device(const uint64_t *rp, const uint32_t *ci, uint64_t n, uint32_t *perm,
-                                    uint32_t *core, int sms, uint64_t *rounds);
+cudaError_t degeneracy_order_device(const uint64_t *rp, const uint32_t *ci, uint64_t n, uint64_t m, uint32_t *perm,
+                                    uint32_t *core, int sms, uint64_t *launches);
 // The CSR with vertex v renamed perm[v], rows sorted (kcore.cu); synchronous.
 // new_rp (n+1) and new_ci (m) are allocated here (cudaMalloc); rows are sorted
 // in calls of at most max_chunk entries (a row longer than that: NotSupported).

@@ -1063,14 +1063,14 @@ int g2_degeneracy_order_device(g2_ctx *ctx, uint32_t *perm, uint32_t *core) {
     uint32_t *d_perm = nullptr, *d_core = nullptr;
     G2_TRY(cudaMalloc(&d_perm, n * 4));
     cudaError_t e = cudaMalloc(&d_core, n * 4);
-    uint64_t rounds = 0;
-    if (e == cudaSuccess) e = g2::degeneracy_order_device(ctx->d_rp, ctx->d_ci, n, d_perm, d_core, ctx->sm_count, &rounds);
+    uint64_t launches = 0;
+    if (e == cudaSuccess) e = g2::degeneracy_order_device(ctx->d_rp, ctx->d_ci, n, ctx->m, d_perm, d_core, ctx->sm_count, &launches);
     if (e == cudaSuccess) e = cudaMemcpy(perm, d_perm, n * 4, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && core) e = cudaMemcpy(core, d_core, n * 4, cudaMemcpyDeviceToHost);
     cudaFree(d_perm);
     cudaFree(d_core);
     if (e != cudaSuccess) return fail_cuda(ctx, e, "degeneracy_order_device");
-    ctx->launches = 2 * rounds + 4;
+    ctx->launches = launches;
     return G2_OK;
 }
 
@@ -1088,11 +1088,11 @@ int g2_degeneracy_recode_device(g2_ctx *ctx, uint32_t *perm, uint32_t *core) {
     uint32_t *d_perm = nullptr, *d_core = nullptr;
     uint64_t *nrp = nullptr;
     uint32_t *nci = nullptr;
-    uint64_t rounds = 0;
+    uint64_t launches = 0;
     cudaError_t e = cudaMalloc(&d_perm, n * 4);
     if (e == cudaSuccess) e = cudaMalloc(&d_core, n * 4);
     if (e == cudaSuccess)
-        e = g2::degeneracy_order_device(ctx->d_rp, ctx->d_ci, n, d_perm, d_core, ctx->sm_count, &rounds);
+        e = g2::degeneracy_order_device(ctx->d_rp, ctx->d_ci, n, ctx->m, d_perm, d_core, ctx->sm_count, &launches);
     if (e == cudaSuccess) e = g2::recode_device(ctx->d_rp, ctx->d_ci, n, m, d_perm, max_chunk, ctx->sm_count, &nrp, &nci);
     if (e == cudaSuccess && perm) e = cudaMemcpy(perm, d_perm, n * 4, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && core) e = cudaMemcpy(core, d_core, n * 4, cudaMemcpyDeviceToHost);
@@ -1125,7 +1125,7 @@ int g2_degeneracy_recode_device(g2_ctx *ctx, uint32_t *perm, uint32_t *core) {
     cudaFree(d_core);
     if (rc) return rc;
     ctx->core_loaded = true;
-    ctx->launches = 2 * rounds + 12;
+    ctx->launches = launches + 12;
     return G2_OK;
 }
 
