@@ -9,17 +9,23 @@
 //  1. clique_prepare_kernel writes the bit matrix of the graph's dense core
 //     (g2_corebits.cuh) and drops the tasks whose root cannot hold a clique
 //     (|P0| < k - 1; two thirds of the roots of R-MAT s20), listing the others.
-//  2. clique_kernel, a persistent grid, builds each root's upper rows 32
-//     candidates per load and ballot and counts pairs of rows by AND + popc.
+//  2. clique_kernel, a persistent grid, builds each root's rows 32 heads
+//     by 32 columns at a time and counts pairs of rows by AND + popc.
 //
 // How a root is walked depends on p = |P0|:
 //   p <= 32          one warp, a row per lane in registers;
 //   p <= kWarpP      one warp, rows in the warp's shared memory;
 //   larger, ordered  the CTA's warps share the root: rows in the CTA's shared
-//                    memory, depth-1 vertices taken from a shared counter;
+//                    memory, chunks of work taken from a shared counter (for
+//                    5-cliques from 65 vertices on: 2.5 -> 1.7 ms on R-MAT s16);
 //   larger, in order one warp, rows in the warp's slab (runs in the caller's
 //                    order, which take the roots one by one as given).
-// Rows are stored as a packed triangle (row i keeps words i / 32 .. W - 1, at
+// Measured (B200, forward lists and one warp per root -> this): 4-cliques of R-MAT
+// s20 15.3 -> 3.6 ms (13.1 -> 2.5 G warp instructions; logic pipe and probe
+// latency bound it), triangles of s18 6.1 -> 0.28 ms, 5-cliques of s16 31 -> 1.5 ms.
+// A warp per root for all widths in schedule order was slower (5.2 ms on s20: the
+// heavy roots' rows fight for the L1), fewer than 8 warps per CTA too (5.4 ms).
+// Rows are stored as a packed triangle (row i keeps words 0 .. i / 32, at
 // an odd stride so that lanes reading rows of one tile hit different banks),
 // which halves the shared memory of a root: p = 658 takes 31 KB, so five CTAs of
 // 8 warps stay resident.
@@ -600,6 +606,13 @@ __device__ __forceinline__ void core_rows(const CoreBits &c, const uint64_t *rp,
     }
 }
 
+__global__ void __launch_bounds__(256) core_rows_kernel(const __grid_constant__ CoreBits c, const uint64_t *rp,
+                                                        const uint32_t *ci, const uint32_t *fo, uint32_t *out) {
+    __shared__ __align__(16) uint32_t seg_all[8][kSeg];
+    core_rows(c, rp, ci, fo, out, seg_all[threadIdx.x >> 5],
+              ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, ((uint64_t)gridDim.x * blockDim.x) >> 5);
+}
+
 // The task lists and the core's bit rows.
 __global__ void __launch_bounds__(256) clique_prepare_kernel(const __grid_constant__ CliqueArgs a, uint32_t k) {
     __shared__ __align__(16) uint32_t seg_all[8][kSeg];
@@ -704,6 +717,13 @@ int clique_blocks_per_sm(uint32_t k, bool in_order, int wpb, uint32_t smem_words
         case 5: return in_order ? clique_occ<5, true>(wpb, sm) : clique_occ<5, false>(wpb, sm);
         default: return 0;
     }
+}
+
+cudaError_t core_rows_launch(const CoreBits &core, uint32_t *bits, const uint64_t *rp, const uint32_t *ci,
+                             const uint32_t *fo, int sms, cudaStream_t st) {
+    const uint64_t blocks = ((uint64_t)core.rows + 7) / 8, cap = 8ull * (uint64_t)sms;
+    if (blocks) core_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(core, rp, ci, fo, bits);
+    return cudaGetLastError();
 }
 
 cudaError_t clique_prepare_launch(const CliqueArgs &a, uint32_t k, int sms, cudaStream_t st) {

@@ -45,7 +45,9 @@ struct Csr {
 // heads), heads = the first nh lanes' `hid`; on return bit i of a lane's word
 // says whether its column is a forward neighbour of head i.  Bits of columns
 // that do not come after the head in P0 are unspecified (the caller masks
-// them).  Lanes beyond P0 pass any id of P0 and mask their word.
+// them).  Lanes beyond P0 pass any id of P0 and mask their word.  With LISTS =
+// false the bits of heads without a bit row stay 0 (see list_rows).
+template <bool LISTS = true>
 __device__ __forceinline__ uint32_t core_tile(const Csr &g, const CoreBlock &b, uint32_t hid, uint32_t nh,
                                               uint32_t cid) {
     const uint32_t nout = __popc(__ballot_sync(G2_FULL, hid < b.base) & (nh >= 32u ? G2_FULL : (1u << nh) - 1u));
@@ -72,7 +74,7 @@ __device__ __forceinline__ uint32_t core_tile(const Csr &g, const CoreBlock &b, 
     // heads without a bit row come first (ids are sorted): four binary searches
     // in step, so that four loads are in flight
     uint32_t h = 0;
-    for (; h < nout; h += 4) {
+    for (; LISTS && h < nout; h += 4) {
         const uint32_t *list[4];
         uint32_t len[4], pos[4], most = 0;
 #pragma unroll
@@ -106,6 +108,32 @@ __device__ __forceinline__ uint32_t core_tile(const Csr &g, const CoreBlock &b, 
     }
     for (; h < nh; h++) acc = __funnelshift_r(acc, word(h) >> (c & 31u), 1);
     return nh >= 32u ? acc : acc >> (32u - nh);
+}
+
+// Rows over P0 (ids, p of them) of up to 32 heads before P0, a lane each, from
+// their forward lists: put(j) sets bit j of the lane's row.  For heads without a
+// bit row that come in numbers (back neighbours of the dense core: short lists,
+// which 32 lanes read at once where core_tile would search them four at a time).
+template <class F>
+__device__ __forceinline__ void list_rows(const Csr &g, const uint32_t *ids, uint32_t p, uint32_t head, bool on, F put) {
+    if (on) {
+        const uint32_t first = ids[0], last = ids[p - 1u];
+        const uint64_t end = ldg(g.rp + head + 1);
+        uint64_t e = lower_bound(g.ci, ldg(g.rp + head) + ldg(g.fo + head), end, first);
+        uint32_t j = 0;
+        for (; e < end && j < p; e++) {
+            const uint32_t y = ldg(g.ci + e);
+            if (y > last) break;
+            uint32_t hi = p;
+            while (j < hi) {
+                const uint32_t mid = (j + hi) >> 1;
+                if (ids[mid] < y) j = mid + 1;
+                else hi = mid;
+            }
+            if (j < p && ids[j] == y) put(j);
+        }
+    }
+    __syncwarp();
 }
 
 }  // namespace g2

@@ -28,6 +28,11 @@ __device__ __forceinline__ unsigned long long vload(const unsigned long long *p)
 }
 __device__ __forceinline__ uint32_t vload32(const uint32_t *p) { return *reinterpret_cast<const volatile uint32_t *>(p); }
 
+// The run's epoch (constant during the kernel; kept out of the argument block,
+// which would otherwise be copied to local memory by every thread).
+template <class Args>
+__device__ __forceinline__ uint32_t run_epoch(const Args &a) { return a.epoch_dev ? __ldcg(a.epoch_dev) : a.epoch; }
+
 // Reserve n consecutive records with one atomic (no retries: many warps hand
 // off work at the same moment).  The slots that exist are added to the
 // outstanding count before any of them is published (the caller is itself
@@ -48,8 +53,9 @@ __device__ __forceinline__ unsigned long long reserve_records(const Args &a, uin
         a.records[i * a.rec_stride + 1] = kVoidRecord;
     __syncwarp();
     __threadfence();
+    const uint32_t epoch = run_epoch(a);
     for (unsigned long long i = base + lane_id(); i < a.rec_cap && i < base + n; i += 32)
-        *reinterpret_cast<volatile uint32_t *>(a.ready + i) = a.epoch;
+        *reinterpret_cast<volatile uint32_t *>(a.ready + i) = epoch;
     __syncwarp();
     return ~0ull;
 }
@@ -60,8 +66,9 @@ template <class Args>
 __device__ __forceinline__ void publish_records(const Args &a, unsigned long long k0, unsigned long long k1) {
     __syncwarp();
     __threadfence();
+    const uint32_t epoch = run_epoch(a);
     for (unsigned long long i = k0 + lane_id(); i < k1; i += 32)
-        *reinterpret_cast<volatile uint32_t *>(a.ready + i) = a.epoch;
+        *reinterpret_cast<volatile uint32_t *>(a.ready + i) = epoch;
     __syncwarp();
 }
 
@@ -83,30 +90,50 @@ __device__ __forceinline__ void outstanding_add(const Args &a, bool on, long lon
     }
 }
 
+// What a CTA's waiting warps know of the queue.  Thousands of waiting warps that
+// poll the shared counters themselves slow the walks down (R-MAT s16 plan walks:
+// 8.7 s with sleeps up to 2 us, 6.6 s with 16 us) or, asleep for longer, leave
+// late and answer late (maximal cliques of G(2000, .01): 114 us, most of it the
+// last sleep).  One warp of the CTA reads the counters, at most every
+// Args::kPollCycles, and the others look at shared memory between sleeps of up to
+// Args::kMaxSleepNs (the walks of plans are longer and fill the SM: less often).
+struct QueueWatch {
+    unsigned long long nrec;  // records reserved, as of the last look
+    unsigned int last;        // clock of the last look
+    unsigned int done;        // no work outstanding
+};
+
+// Before any warp of the CTA waits (a CTA barrier must follow).
+__device__ __forceinline__ void watch_init(QueueWatch *q) {
+    if (threadIdx.x == 0) {
+        q->nrec = 0;
+        q->last = (unsigned int)clock64();
+        q->done = 0;
+    }
+}
+
 // Phase 2 of a pass that hands off work: take tickets and run their records
 // (run(h) runs record h) until no work is outstanding.
-// Backoff cap of a waiting warp.  Thousands of waiting warps poll; with a 2 us
-// cap their traffic on the counters' L2 slice slowed the warps still working
-// (plan walks on R-MAT s16: 8.7 s -> 6.6 s with 16 us), with no loss for MCE.
-constexpr uint32_t kMaxSleepNs = 16384;
-
 template <class Args, class Run>
-__device__ void run_record_queue(const Args &a, Run run) {
-    const uint32_t lane = lane_id();
+__device__ void run_record_queue(const Args &a, QueueWatch *watch, Run run) {
+    volatile QueueWatch *q = watch;
+    const uint32_t lane = lane_id(), epoch = run_epoch(a);
     unsigned long long h = 0;
     if (lane == 0) h = atomicAdd(a.qctl + kQHead, 1ull);
     h = __shfl_sync(G2_FULL, h, 0);
-    uint32_t sleep_ns = 32, polls = 0;
+    uint32_t sleep_ns = 32;
     long long w0 = clock64();
     for (;;) {
         int action = 0;  // 0 wait, 1 run record h, 2 leave
         if (lane == 0) {
-            if (h < a.rec_cap && vload32(a.ready + h) == a.epoch) {
-                action = 1;
-            } else if ((++polls & 3u) == 0) {  // the shared counter on every 4th poll only
+            const unsigned int now = (unsigned int)clock64(), last = q->last;
+            if (now - last > Args::kPollCycles && atomicCAS(&watch->last, last, now) == last) {
                 __threadfence();  // whatever this warp saw taken was counted first
-                if (vload(a.qctl + kQOut) == 0) action = 2;
+                if (vload(a.qctl + kQOut) == 0) q->done = 1;
+                q->nrec = vload(a.nrec);
             }
+            if (h < q->nrec && h < a.rec_cap && vload32(a.ready + h) == epoch) action = 1;
+            else if (q->done) action = 2;
         }
         action = __shfl_sync(G2_FULL, action, 0);
         if (action == 1) {
@@ -127,7 +154,7 @@ __device__ void run_record_queue(const Args &a, Run run) {
             break;
         }
         __nanosleep(sleep_ns);
-        sleep_ns = sleep_ns < kMaxSleepNs ? sleep_ns * 2 : kMaxSleepNs;
+        sleep_ns = sleep_ns < Args::kMaxSleepNs ? sleep_ns * 2 : Args::kMaxSleepNs;
     }
 }
 

@@ -44,6 +44,7 @@ struct CoreBits {
 CoreBlock core_block_of(uint32_t lo, uint32_t n, uint64_t bytes, uint32_t row0, uint64_t off);
 
 struct MceArgs {
+    static constexpr uint32_t kPollCycles = 6000, kMaxSleepNs = 4096;  // of waiting warps (g2_handoff.cuh)
     const uint64_t *rp;
     const uint32_t *ci;
     const uint32_t *fo;             // fo[v]: offset in N(v) of the first neighbour > v
@@ -55,7 +56,7 @@ struct MceArgs {
     uint64_t ntasks;                // tasks in this pass (if ntasks_dev is null)
     const unsigned long long *ntasks_dev;  // else: task count read from device memory
     unsigned long long *head;       // device queue head
-    uint32_t chunk;                 // tasks grabbed per atomic
+    uint32_t chunk;                 // tasks grabbed per atomic (0: 1, more among the light tasks)
     uint32_t hist_len;
     uint32_t *scratch;              // warps * words_per_warp words
     uint64_t words_per_warp;        // multiple of 64
@@ -86,6 +87,8 @@ struct MceArgs {
     uint64_t wait_cycles;           // longest wait of a warp for its ticket's record
     const unsigned long long *deadline;  // optional: %globaltimer (ns) past which roots are
                                          // dropped (set on the device by deadline_set)
+    CoreBits core;                  // bit rows (core.bits null: every root takes the general walk)
+    uint32_t sorted;                // tasks in descending cost (chunk 0)
 };
 constexpr int kQHead = 0, kQOut = 1;
 constexpr uint32_t kMatchRecordWords = 32;  // stride of a plan-walk record
@@ -128,6 +131,7 @@ struct DevPlan {
 };
 
 struct MatchArgs {
+    static constexpr uint32_t kPollCycles = 24000, kMaxSleepNs = 16384;  // of waiting warps (g2_handoff.cuh)
     const uint64_t *rp;
     const uint32_t *ci;
     const uint32_t *fo;
@@ -210,6 +214,9 @@ uint32_t clique_p_fit(uint32_t k, bool in_order, uint64_t words_per_warp, int wa
 // Dynamic shared memory (words) for roots up to max_fwd, and a row's word count for 5-cliques.
 uint32_t clique_smem_words(uint32_t k, bool in_order, uint32_t max_fwd, int warps_per_block, uint32_t *q_words);
 int clique_blocks_per_sm(uint32_t k, bool in_order, int warps_per_block, uint32_t smem_words);
+// The core's bit rows alone (core.bits), in stream order.
+cudaError_t core_rows_launch(const CoreBits &core, uint32_t *bits, const uint64_t *rp, const uint32_t *ci,
+                             const uint32_t *fo, int sms, cudaStream_t st);
 cudaError_t clique_prepare_launch(const CliqueArgs &a, uint32_t k, int sms, cudaStream_t st);
 cudaError_t clique_launch(const CliqueArgs &a, uint32_t k, int blocks, int warps_per_block, cudaStream_t st);
 

@@ -888,7 +888,9 @@ template <int WPL, bool METRICS, int MINB>
 __global__ void __launch_bounds__(256, MINB) match_kernel(MatchArgs a, int clique_path,
                                                           const __grid_constant__ DevPlan pl) {
     extern __shared__ uint32_t smem[];
-    if (a.epoch_dev) a.epoch = *a.epoch_dev;
+    __shared__ QueueWatch watch;
+    watch_init(&watch);
+    __syncthreads();
     const uint32_t wib = threadIdx.x >> 5;
     uint32_t *rowbuf = smem + wib * (32u * WPL + a.p0_words);
     uint32_t *p0s = rowbuf + 32u * WPL;
@@ -938,7 +940,7 @@ __global__ void __launch_bounds__(256, MINB) match_kernel(MatchArgs a, int cliqu
         outstanding_add(a, handoff, -1);
     }
     if (handoff)
-        run_record_queue(a, [&](unsigned long long h) {
+        run_record_queue(a, &watch, [&](unsigned long long h) {
             const uint32_t *rec = a.records + h * a.rec_stride;
             if (__ldcg(rec + 1) == kVoidRecord) return;  // slot of a reservation that did not fit
             long long c0 = 0;

@@ -42,6 +42,7 @@
 #include "g2_device.cuh"
 #include "g2_handoff.cuh"
 #include "g2_kernels.h"
+#include "g2_mce_fast.cuh"
 
 namespace g2 {
 
@@ -335,7 +336,7 @@ __device__ __forceinline__ bool deadline_passed(const MceArgs &a) {
 // sum_{q in P \ N(pivot)} (|P ∪ X| + deg q) for the children.
 template <int WPL, bool METRICS, bool BUDGET>
 __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t *cand, uint32_t *rowbuf,
-                        long long c0, uint32_t *task_out) {
+                        uint32_t *hist, unsigned long long *found, long long c0, uint32_t *task_out) {
     const uint32_t lane = lane_id();
     const uint64_t *rp = a.rp;
     const uint32_t *ci = a.ci;
@@ -381,14 +382,39 @@ __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t 
     const uint32_t W = (p + 31u) >> 5;
     if (W > 32u * WPL) return kTaskDeferred;
     const uint64_t SW = a.words_per_warp;
+    // small roots, and the small branches of the others, take fast_walk
+    constexpr bool kFast = WPL == 1 && !METRICS && !BUDGET;
+    const bool fast = kFast && a.core.bits && nparts == 1;
+    if (kFast && fast && !is_rec && p <= kFastN && kFastSlab <= SW) {
+        FastHead *head = reinterpret_cast<FastHead *>(S);
+        const uint32_t kept = fast_root(a, v, split, p, nx, head, cand);
+        if (kept != ~0u) {
+            const FastSum r = fast_any(a, task, p, p, kept, head, cand, hist, nullptr, c0);
+            if (lane == 0) {
+                if (a.root_nodes) atomicAdd(reinterpret_cast<unsigned long long *>(a.root_nodes + task), r.nodes);
+                if (a.root_cliques && r.cliques)
+                    atomicAdd(reinterpret_cast<unsigned long long *>(a.root_cliques + task), r.cliques);
+            }
+            *found += r.cliques;
+            return kTaskDone;
+        }
+    }
     const uint32_t FR = frame_words(W);
+    // the slab's end holds the general frames, before them (16-byte aligned) a fast walk's state
     const uint64_t fr0 = SW >= (uint64_t)(p + 1) * FR ? SW - (uint64_t)(p + 1) * FR : 0;
+    const uint64_t sub_words = fast ? (kFastSlab + 15u) & ~15u : 0u;
+    // (main pass only: a deferred root has the whole slab for its lists)
+    const bool sub = fast && !a.task_index && (fr0 & ~15ull) >= sub_words + 2ull * (p + 2) + 64;
+    const uint64_t lim = sub ? (fr0 & ~15ull) - sub_words : fr0;  // lists stay below
     unsigned long long *hist_local = a.hist_dev ? a.hist_dev : reinterpret_cast<unsigned long long *>(S);
     const uint64_t a0 = 2ull * (p + 2);  // after the histogram
     // nothing is written before the slab is known to hold the histogram and frames
     // (a small slab's neighbours are other warps' slabs)
-    if (fr0 < a0 + 64) return kTaskDeferred;
+    if (lim < a0 + 64) return kTaskDeferred;
     for (uint32_t s = lane; s < p + 2; s += 32) hist_local[s] = 0ull;
+    uint32_t *hist2 = hist + kFastHist;  // sizes found by this entry's fast walks (kFast)
+    if (kFast && sub)
+        for (uint32_t s = lane; s < kFastHist; s += 32) hist2[s] = 0u;
     Rows rows;
     uint32_t nb;
     uint64_t l0;  // list region
@@ -398,15 +424,20 @@ __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t 
         // slab: [hist u64 (p+2)] [A p*W] [xv nx (metrics)] [B nb*W] [lists ...] ... [frames (p+1)*FR]
         const uint64_t xv0 = a0 + (uint64_t)p * W;
         const uint64_t b0 = xv0 + (METRICS ? nx : 0);
-        if (fr0 < b0 + 64) return kTaskDeferred;
-        // stage P0 in shared memory, then the rows
-        for (uint32_t i = lane; i < p; i += 32) cand[i] = ldg(ci + split + i);
-        __syncwarp();
-        build_forward_rows(rp, ci, a.fo, cand, p, W, S + a0, rowbuf);
+        if (lim < b0 + 64) return kTaskDeferred;
         // kept B rows plus their root-list entries must stay below the frames
-        const uint64_t cap64 = (fr0 - b0 - 64) / (W + 1);
+        const uint64_t cap64 = (lim - b0 - 64) / (W + 1);
         const uint32_t cap = cap64 > 0xfffffff0ull ? 0xfffffff0u : (uint32_t)cap64;
-        nb = build_back_rows(rp, ci, a.fo, v, lo, nx, cand, p, W, S + b0, METRICS ? S + xv0 : nullptr, cap, rowbuf);
+        nb = ~0u;
+        if (!METRICS && a.core.bits) nb = core_rows_of_root(a, v, split, p, nx, S + a0, S + b0, cap, cand);
+        if (nb == ~0u) {  // no bit rows (or barely room): from the forward lists
+            // stage P0 in shared memory, then the rows
+            for (uint32_t i = lane; i < p; i += 32) cand[i] = ldg(ci + split + i);
+            __syncwarp();
+            build_forward_rows(rp, ci, a.fo, cand, p, W, S + a0, rowbuf);
+            nb = build_back_rows(rp, ci, a.fo, v, lo, nx, cand, p, W, S + b0, METRICS ? S + xv0 : nullptr, cap,
+                                 rowbuf);
+        }
         if (nb == ~0u) return kTaskDeferred;
         __syncwarp();
         rows.A = S + a0;
@@ -432,7 +463,7 @@ __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t 
         rows.B = rows.A + (uint64_t)p * W;
         rows.xv = rows.B + (uint64_t)nb * W;
         l0 = a0;
-        if (fr0 < l0 + nb + 64) return kTaskDeferred;
+        if (lim < l0 + nb + 64) return kTaskDeferred;
         row_load_cg(P, rec + kRecRows, W);
         row_load_cg(X, rec + kRecRows + W, W);
         row_load_cg(Rb, rec + kRecRows + 2u * W, W);
@@ -467,6 +498,23 @@ __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t 
     long long next_check = (long long)a.spill_cycles;
     for (;;) {
         bool want_pop = false;
+        if (kFast && enter && sub && xlen <= kFastM && d0 + d < kFastDepth && row_any(P)) {
+            const uint32_t cnt = p <= kFastN ? p : fast_members(P.w[0], X.w[0]);
+            if (cnt <= kFastN) {  // this node's whole branch
+                const Row<WPL> R = path_of<WPL>(S + fr0, d, W, Rb);
+                FastHead *head = reinterpret_cast<FastHead *>(S + lim);
+                fast_sub(p, cnt, P.w[0], X.w[0], R.w[0], d0 + d,
+                         rows.pool_off == ~0ull ? ~0u : (uint32_t)(rows.pool_off >> 6), nb, rows.A, rows.B, S + xoff,
+                         xlen, head, cand);
+                const FastSum r = fast_any(a, task, p, cnt, xlen, head, cand, hist2, hist_local, c0);
+                nodes += r.nodes;
+                cliques += r.cliques;
+                donated = donated || r.donated;
+                if (rows.pool_off == ~0ull && head->unit != ~0u) rows.pool_off = (uint64_t)head->unit << 6;
+                enter = false;
+                want_pop = true;
+            }
+        }
         if (enter) {
             enter = false;
             if (BUDGET && (nodes & 255u) == 0 && deadline_passed(a)) {  // time budget: drop the root
@@ -605,7 +653,7 @@ __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t 
                 row_assign_bit(Qr, q, false);
                 if (d + 1 == D && (branch++ % nparts) != part) continue;  // another part's subtree
                 const uint64_t coff = xoff + xlen;
-                if (coff + xlen > fr0) {         // child list would reach the frames
+                if (coff + xlen > lim) {         // child list would reach the frames
                     if (may_spill || donated) {  // hand this level and the ones below to records
                         Row<WPL> P1 = P, X1 = X, Q1 = Qr;
                         row_assign_bit(P1, q, true);
@@ -678,6 +726,7 @@ __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t 
         if (lane == 0) atomicOr(a.status, kStatusDeferOverflow);  // record buffers full: incomplete
     }
     // ---- commit this entry's results
+    if (kFast && sub) fast_keep(hist2, hist_local, p + 2u < kFastHist ? p + 2u : kFastHist);
     __syncwarp();
     if (lane == 0) {
         atomicAdd(a.out, cliques);
@@ -699,15 +748,22 @@ __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t 
 
 template <int WPL, bool METRICS, bool BUDGET>
 __device__ __forceinline__ void run_entry(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t *cand,
-                                          uint32_t *rowbuf) {
+                                          uint32_t *rowbuf, uint32_t *hist, unsigned long long *found) {
     long long c0 = 0;
     if (lane_id() == 0) c0 = clock64();
     c0 = __shfl_sync(G2_FULL, c0, 0);
     uint32_t task = 0;
-    if (mce_task<WPL, METRICS, BUDGET>(a, entry, S, cand, rowbuf, c0, &task) == kTaskDeferred)
+    if (mce_task<WPL, METRICS, BUDGET>(a, entry, S, cand, rowbuf, hist, found, c0, &task) == kTaskDeferred)
         defer_entry(a, entry);
     else if (a.root_cost && lane_id() == 0 && task != ~0u)
         atomicAdd(reinterpret_cast<unsigned long long *>(a.root_cost + task), (unsigned long long)(clock64() - c0));
+}
+
+// Shared memory of a warp (words): candidates and a row buffer, or fast_walk's
+// rows; then the sizes its walks have found.
+__host__ __device__ constexpr uint32_t mce_warp_words(uint32_t wpl) {
+    const uint32_t general = 32u * 32u * wpl + 32u * wpl;
+    return wpl > 1 ? general : (general > kFastArea ? general : kFastArea) + 2u * kFastHist;
 }
 
 // Persistent pass.  Phase 1: entries from the task queue (or a deferred list).
@@ -716,12 +772,18 @@ __device__ __forceinline__ void run_entry(const MceArgs &a, uint32_t entry, uint
 // BUDGET: the build for runs with a time budget (MceArgs::deadline set); the
 // others carry no deadline check.
 template <int WPL, bool METRICS, bool BUDGET>
-__global__ void __launch_bounds__(256, 3) mce_kernel(MceArgs a) {
+__global__ void __launch_bounds__(256, 3) mce_kernel(const __grid_constant__ MceArgs a) {
     extern __shared__ uint32_t smem[];
-    if (a.epoch_dev) a.epoch = *a.epoch_dev;
+    __shared__ QueueWatch watch;
+    watch_init(&watch);
+    __syncthreads();
     const uint32_t wib = threadIdx.x >> 5;
-    uint32_t *cand = smem + wib * (32u * 32u * WPL + 32u * WPL);
+    uint32_t *cand = smem + wib * mce_warp_words(WPL);
     uint32_t *rowbuf = cand + 32u * 32u * WPL;
+    uint32_t *hist = cand + mce_warp_words(WPL) - 2u * kFastHist;  // sizes found by roots' fast walks, and an entry's
+    unsigned long long found = 0;                             // cliques found by fast_walk
+    if (WPL == 1)
+        for (uint32_t s = lane_id(); s < kFastHist; s += 32) hist[s] = 0;
     const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     uint32_t *S = a.scratch + gw * a.words_per_warp;
     const bool handoff = a.spill_cycles != 0;
@@ -730,33 +792,42 @@ __global__ void __launch_bounds__(256, 3) mce_kernel(MceArgs a) {
         n = *a.ntasks_dev;
         if (n > a.deferred_cap) n = a.deferred_cap;
     }
+    // a warp is outstanding from before its first task until it has done its last
+    // (counted once: three atomics on shared words per task cost more than a light root)
+    outstanding_add(a, handoff, 1);
+    uint32_t chunk = a.chunk ? a.chunk : 1u;
     for (;;) {
-        outstanding_add(a, handoff, 1);
-        const unsigned long long t0 = grab(a.head, a.chunk);
-        if (t0 >= n) {
-            outstanding_add(a, handoff, -1);
-            break;
-        }
-        const unsigned long long t1 = t0 + a.chunk < n ? t0 + a.chunk : n;
+        const unsigned long long t0 = grab(a.head, chunk);
+        if (t0 >= n) break;
+        const unsigned long long t1 = t0 + chunk < n ? t0 + chunk : n;
+        // heavy tasks one at a time, light ones several per atomic: the light end
+        // is the last seven eighths of a cost-ordered list, or the first three
+        // quarters of one in the given (degeneracy) order
+        if (!a.chunk) chunk = a.sorted ? (t0 * 8 > n ? 8u : 1u) : (t0 * 4 < n * 3 ? 4u : 1u);
         for (unsigned long long t = t0; t < t1; t++) {
             if (BUDGET && deadline_passed(a)) {  // time budget spent: start no new root
                 if (lane_id() == 0) atomicOr(a.status, kStatusDeadline);
                 continue;
             }
-            run_entry<WPL, METRICS, BUDGET>(a, a.task_index ? a.task_index[t] : (uint32_t)t, S, cand, rowbuf);
+            run_entry<WPL, METRICS, BUDGET>(a, a.task_index ? a.task_index[t] : (uint32_t)t, S, cand, rowbuf, hist,
+                                            &found);
         }
-        outstanding_add(a, handoff, -1);
     }
+    outstanding_add(a, handoff, -1);
     if (handoff)
-        run_record_queue(a, [&](unsigned long long h) {
-            run_entry<WPL, METRICS, BUDGET>(a, kRecordBit | (uint32_t)h, S, cand, rowbuf);
+        run_record_queue(a, &watch, [&](unsigned long long h) {
+            run_entry<WPL, METRICS, BUDGET>(a, kRecordBit | (uint32_t)h, S, cand, rowbuf, hist, &found);
         });
+    if (WPL == 1) {
+        fast_flush(a, hist);
+        if (lane_id() == 0 && found) atomicAdd(a.out, found);
+    }
 }
 
 }  // namespace
 
 size_t mce_smem_bytes(int wpl, int warps_per_block) {
-    return (size_t)warps_per_block * (32u * 32u * wpl + 32u * wpl) * sizeof(uint32_t);
+    return (size_t)warps_per_block * mce_warp_words((uint32_t)wpl) * sizeof(uint32_t);
 }
 
 template <int WPL, bool M>

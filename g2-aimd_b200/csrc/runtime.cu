@@ -647,13 +647,25 @@ int mce_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned long
         ctx->launches++;
         base.deadline = ctx->d_deadline;
     }
+    base.sorted = o && o->schedule != G2_SCHED_GIVEN;
+    if (!base.work && !deadline_ms && !tl.split) {  // (those runs take the general walk)
+        rc = ensure_clique(ctx, 0, st, &base.core);
+        if (rc && rc != G2_ERR_OOM) return rc;
+        if (rc) base.core.bits = nullptr;
+    }
     if (ctx->timed) G2_TRY(cudaEventRecord(ctx->ev[0], st));
     L2Window l2(ctx, st, flags);
+    if (base.core.bits) {
+        cudaError_t e = g2::core_rows_launch(base.core, ctx->d_core_bits, ctx->d_rp, ctx->d_ci, ctx->d_fo,
+                                             ctx->sm_count, st);
+        if (e != cudaSuccess) return fail_cuda(ctx, e, "core_rows_launch");
+        ctx->launches++;
+    }
     {  // main pass: every task, WPL=1, one slab per resident warp; long walks
        // hand branches to idle warps through the record queue
         g2::MceArgs a = base;
         a.head = ctx->d_ctr + kCtrHead;
-        a.chunk = (o && o->chunk) ? o->chunk : 1u;
+        a.chunk = o ? o->chunk : 0u;
         a.words_per_warp = (ctx->scratch_words / ((uint64_t)blocks * wpb)) & ~63ull;
         a.deferred = ctx->d_defer;
         a.ndeferred = ctx->d_ctr + kCtrDefer;

@@ -126,7 +126,8 @@ typedef struct g2_opts {
                                    at this search-tree depth (0 = default 2)         */
     uint64_t *root_cost;        /* optional host out: SM cycles per source (summed
                                    over its split tasks)                            */
-    uint32_t chunk;             /* tasks taken per queue atomic (0 = 1 MCE, 4 match) */
+    uint32_t chunk;             /* tasks taken per queue atomic (0 = 1, MCE more among
+                                   its light tasks; 4 for plan walks)               */
     uint32_t spill_kcycles;     /* MCE and plan walks of non-clique plans: every this
                                    many thousand SM cycles a walk checks for idle
                                    warps and hands them the pending work of its

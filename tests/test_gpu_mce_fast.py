@@ -1,0 +1,51 @@
+"""Maximal cliques of roots around the limits of the register walk
+(csrc/g2_mce_fast.cuh): |P0| of 32, 64 and 96, 128 live back rows, branches that
+are renumbered, hand-off on and off; counts, histogram and per-root search-tree
+nodes equal the oracle's."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _layers(g2, sizes, keep, backs, seed):
+    """Random cores of the given sizes (edge probability keep) on the last ids, and
+    `backs` earlier vertices per core, each adjacent to a random third of it."""
+    rng = np.random.default_rng(seed)
+    edges, n = [], sum(backs for _ in sizes)
+    base, x = n, 0
+    for p in sizes:
+        a, b = np.triu_indices(p, 1)
+        on = rng.random(a.size) < keep
+        edges += [(base + int(i), base + int(j)) for i, j in zip(a[on], b[on])]
+        for _ in range(backs):
+            nb = np.flatnonzero(rng.random(p) < 0.33)
+            edges += [(x, base + int(j)) for j in nb]
+            x += 1
+        base += p
+    return g2.Graph.from_edges(base, edges)
+
+
+@pytest.mark.parametrize("keep,backs", [(0.3, 3), (0.3, 200), (0.6, 40)])
+def test_root_sizes(g2, orc, ctx, keep, backs):
+    sizes = [5, 32, 33, 64, 65] + ([96, 97, 130] if keep < 0.5 else [])
+    g = _layers(g2, sizes, keep, backs, 7)
+    want = orc.mce(g, threads=8, per_root=True)
+    ctx.load(g)
+    for kw in ({}, {"schedule": "heuristic"}, {"spill_kcycles": 1}, {"flags": 16}, {"chunk": 3}):
+        c, h, rn = ctx.mce(root_nodes=True, **kw)
+        assert c == want["count"], (keep, backs, kw)
+        assert np.array_equal(h, want["hist"][:h.size]) and np.array_equal(rn, want["root_nodes"]), (keep, backs, kw)
+
+
+def test_sources_and_small_slab(g2, orc):
+    """A subset of the roots, and slabs too small for the register walk's frames."""
+    from g2aimd.context import Context
+    g = g2.Graph.rmat(10, 16, seed=4).degeneracy_recoded()
+    src = np.arange(g.n - 1, -1, -3, dtype=np.uint32)
+    want = orc.mce(g, roots=src, threads=8)
+    for scratch in (0, 148 * 24 * 1024 * 4):
+        with Context(0, scratch_bytes=scratch) as c:
+            c.load(g)
+            cnt, h = c.mce(sources=src)
+            assert cnt == want["count"] and np.array_equal(h, want["hist"][:h.size]), scratch
