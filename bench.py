@@ -608,8 +608,8 @@ def headline_profile():
     """Figures of the headline kernel's ncu capture committed under profiles/
     (R-MAT s20 ef16 seed 1, 4-cliques): DRAM bytes per launch and warp
     instructions per launch."""
-    path = os.path.join(ROOT, "profiles", "match_kernel_k4_rmat_s20.md")
-    out = {"file": "profiles/match_kernel_k4_rmat_s20.md"}
+    path = os.path.join(ROOT, "profiles", "clique_kernel_k4_rmat_s20.md")
+    out = {"file": "profiles/clique_kernel_k4_rmat_s20.md"}
     try:
         text = open(path).read()
     except OSError:
@@ -1054,7 +1054,7 @@ def run_ours(a):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None,
                          "traffic": prof.get("traffic"),
-                         "kernel": "match_kernel<1,0,6> (clique bitmap path), main pass", "kernel_ms": kern_ms,
+                         "kernel": "clique_prepare_kernel + clique_kernel<4,0> (core bit rows), main pass", "kernel_ms": kern_ms,
                          "algorithmic_bytes": stream_bytes, "peak_kind": peak_kind,
                          "binding": "instruction issue (see issue.frac); the HBM fraction is far from binding",
                          "issue": issue,
