@@ -737,6 +737,11 @@ cudaError_t clique_prepare_launch(const CliqueArgs &a, uint32_t k, int sms, cuda
     return cudaGetLastError();
 }
 
+cudaError_t clique_preload() {
+    cudaFuncAttributes fa;
+    return cudaFuncGetAttributes(&fa, clique_prepare_kernel);
+}
+
 template <int K, bool O>
 static void clique_go(const CliqueArgs &a, int blocks, int wpb, cudaStream_t st) {
     const size_t sm = 4ull * a.smem_words;

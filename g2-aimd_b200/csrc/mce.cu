@@ -862,6 +862,17 @@ int mce_blocks_per_sm(int wpl, int warps_per_block, bool metrics) {
     }
 }
 
+cudaError_t mce_preload(int wpl) {
+    cudaFuncAttributes fa;
+    switch (wpl) {
+        case 1: return cudaFuncGetAttributes(&fa, mce_kernel<1, false, true>);
+        case 2: return cudaFuncGetAttributes(&fa, mce_kernel<2, false, true>);
+        case 4: return cudaFuncGetAttributes(&fa, mce_kernel<4, false, true>);
+        case 8: return cudaFuncGetAttributes(&fa, mce_kernel<8, false, true>);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 __global__ void epoch_bump_kernel(uint32_t *e) {
     uint32_t v = *e + 1u;
     *e = v ? v : 1u;

@@ -642,7 +642,10 @@ int mce_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned long
     base.epoch_dev = spill ? ctx->d_epoch : nullptr;
     base.wait_cycles = (o && o->wait_cycles) ? o->wait_cycles : kWaitCycles;
     if (deadline_ms) {
-        cudaError_t e = g2::deadline_set(ctx->d_deadline, 1000000ull * deadline_ms, st);
+        // the budget starts on the device: the kernels' code is loaded before it does
+        cudaError_t e = g2::mce_preload(1);
+        if (e == cudaSuccess) e = g2::mce_preload(wpl_for(ctx->max_fwd));
+        if (e == cudaSuccess) e = g2::deadline_set(ctx->d_deadline, 1000000ull * deadline_ms, st);
         if (e != cudaSuccess) return fail_cuda(ctx, e, "deadline_set");
         ctx->launches++;
         base.deadline = ctx->d_deadline;
@@ -868,12 +871,7 @@ int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned lo
     a.work = (flags & G2_FLAG_WORK_MODEL) ? ctx->d_work : nullptr;
     const bool clique = ctx->clique_plan && !(o && o->intersect_mode == 1);
     const uint32_t deadline_ms = o ? o->deadline_ms : 0u;
-    if (deadline_ms) {  // time budget: unfinished roots are dropped whole, so no hand-off
-        cudaError_t ed = g2::deadline_set(ctx->d_deadline, 1000000ull * deadline_ms, st);
-        if (ed != cudaSuccess) return fail_cuda(ctx, ed, "deadline_set");
-        ctx->launches++;
-        a.deadline = ctx->d_deadline;
-    }
+    if (deadline_ms) a.deadline = ctx->d_deadline;  // unfinished roots are dropped whole, so no hand-off
     // plan walks (non-clique plans) hand pending work to idle warps
     if (!clique && !(flags & G2_FLAG_NO_SPILL) && !deadline_ms) {
         rc = ensure_handoff(ctx, st);
@@ -929,6 +927,12 @@ int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned lo
         q.root_cost = d_root_cost;
         q.status = ctx->d_status;
         q.deadline = a.deadline;
+    }
+    if (deadline_ms) {  // the budget starts on the device: the kernels' code has been loaded before it does
+        cudaError_t ed = rows ? g2::clique_preload() : cudaSuccess;
+        if (ed == cudaSuccess) ed = g2::deadline_set(ctx->d_deadline, 1000000ull * deadline_ms, st);
+        if (ed != cudaSuccess) return fail_cuda(ctx, ed, "deadline_set");
+        ctx->launches++;
     }
     if (ctx->timed) G2_TRY(cudaEventRecord(ctx->ev[0], st));
     L2Window l2(ctx, st, flags);
