@@ -82,15 +82,21 @@ __device__ __forceinline__ uint32_t flip32(uint32_t x) {
     return x;
 }
 
+// Counts of cliques of `size` vertices to a 64-bit counter: a root's own (which its
+// commit adds to the run's) or the run's.
+__device__ __forceinline__ void fast_count(const MceArgs &a, unsigned long long *keep, uint32_t size, uint32_t h) {
+    if (keep) keep[size] += h;
+    else if (size < a.hist_len) atomicAdd(a.out + 1 + size, (unsigned long long)h);
+    else if (a.hist_len) atomicOr(a.status, kStatusHistOverflow);  // hist_len 0: no histogram
+}
+
 // The clique sizes a warp has found so far (shared memory) to the run's histogram.
 __device__ __noinline__ void fast_flush(const MceArgs &a, uint32_t *hist) {
     __syncwarp();
     for (uint32_t s = lane_id(); s < kFastHist; s += 32) {
         const uint32_t h = hist[s];
         hist[s] = 0;
-        if (!h) continue;
-        if (s < a.hist_len) atomicAdd(a.out + 1 + s, (unsigned long long)h);
-        else if (a.hist_len) atomicOr(a.status, kStatusHistOverflow);  // hist_len 0: no histogram
+        if (h) fast_count(a, nullptr, s, h);
     }
     __syncwarp();
 }
@@ -498,9 +504,16 @@ __device__ __noinline__ FastSum fast_walk(const MceArgs &a, uint32_t task, uint3
         next_check = __shfl_sync(G2_FULL, next_check, 0) / (long long)a.spill_cycles * (long long)a.spill_cycles +
                      (long long)a.spill_cycles;
     }
-    auto found = [&](uint32_t size) {  // a maximal clique of `size` vertices
+    // a maximal clique of `size` vertices; the counters hold 32 bits and live for many
+    // walks, so a full one is emptied on the spot
+    const uint32_t full = a.hist_fold;
+    auto found = [&](uint32_t size) {
         cliques++;
-        if (lane == 0) hist[size]++;
+        if (lane == 0) {
+            const uint32_t h = hist[size] + 1u;
+            hist[size] = h == full ? 0u : h;
+            if (h == full) fast_count(a, keep, size, h);
+        }
     };
     auto save = [&](uint32_t at, uint32_t q) {
         uint32_t f[FW];
@@ -559,10 +572,6 @@ __device__ __noinline__ FastSum fast_walk(const MceArgs &a, uint32_t task, uint3
                 const uint32_t step = best >= nb ? N : M;
 #pragma unroll
                 for (int w = 0; w < W; w++) Q[w] = P[w] & ~row[w * step];
-                if ((nodes & 0xffffffu) == 0) {  // the counters hold 32 bits
-                    if (keep) fast_keep(hist, keep, p + 2u < kFastHist ? p + 2u : kFastHist);
-                    else fast_flush(a, hist);
-                }
                 if (may_spill && (nodes & 15u) == 0) {
                     long long el = 0;
                     if (lane == 0) el = clock64() - c0;

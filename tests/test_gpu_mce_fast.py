@@ -49,3 +49,18 @@ def test_sources_and_small_slab(g2, orc):
             c.load(g)
             cnt, h = c.mce(sources=src)
             assert cnt == want["count"] and np.array_equal(h, want["hist"][:h.size]), scratch
+
+
+@pytest.mark.parametrize("fold", [1, 2, 7])
+def test_size_counters_are_emptied_when_full(g2, orc, ctx, monkeypatch, fold):
+    """The warps' 32-bit size counters live for all roots of a warp: with the count at
+    which they are emptied cut to a few cliques, both those of whole roots and those
+    of branches are crossed many times, and the histogram stays the oracle's."""
+    monkeypatch.setenv("G2_HIST_FOLD", str(fold))
+    for g in (g2.Graph.rmat(11, 16, seed=2).degeneracy_recoded(), _layers(g2, [97, 130], 0.3, 200, 7)):
+        want = orc.mce(g, threads=8)
+        ctx.load(g)
+        for kw in ({}, {"schedule": "heuristic"}, {"flags": 16}):
+            c, h = ctx.mce(**kw)
+            assert c == want["count"] and int(h.sum()) == c, (fold, kw)
+            assert np.array_equal(h, want["hist"][:h.size]), (fold, kw)
