@@ -42,10 +42,10 @@ constexpr uint32_t kFastWords = 3;                // words of a set of vertices
 constexpr uint32_t kFastN = 32u * kFastWords;     // vertices
 constexpr uint32_t kFastB = 4;                    // words of a set of back rows
 constexpr uint32_t kFastM = 32u * kFastB;         // back rows
-constexpr uint32_t kFastHist = 136;               // clique sizes counted in shared memory
-constexpr uint32_t kFastDepth = kFastHist - kFastN - 2u;  // depth from which no size exceeds them
+constexpr uint32_t kFastHist = 104;               // clique sizes counted in shared memory (a small root's all)
 constexpr uint32_t kFastRows = 32u * kFastWords * (kFastWords + 2u * kFastB);  // A, B and B transposed (words)
 constexpr uint32_t kFastArea = kFastRows + kFastN / 2u;   // and the vertices' places in P0
+static_assert(kFastHist >= kFastN + 2u, "a small root's sizes fit");
 constexpr uint32_t kFastRecRows = 4;              // record: [task, depth, pool unit, nb] before P, X, R
 
 template <int W>
@@ -505,11 +505,15 @@ __device__ __noinline__ FastSum fast_walk(const MceArgs &a, uint32_t task, uint3
                      (long long)a.spill_cycles;
     }
     // a maximal clique of `size` vertices; the counters hold 32 bits and live for many
-    // walks, so a full one is emptied on the spot
+    // walks, so a full one is emptied on the spot.  Sizes beyond them (a branch deep in
+    // a large root) go to the root's own: keeping such branches out of this walk
+    // instead made Chung-Lu 2*10^5 (exponent 2.2) 34 ms where it takes 19
     const uint32_t full = a.hist_fold;
     auto found = [&](uint32_t size) {
         cliques++;
-        if (lane == 0) {
+        if (lane == 0 && size >= kFastHist) {
+            keep[size]++;
+        } else if (lane == 0) {
             const uint32_t h = hist[size] + 1u;
             hist[size] = h == full ? 0u : h;
             if (h == full) fast_count(a, keep, size, h);

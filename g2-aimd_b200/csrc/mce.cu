@@ -498,7 +498,7 @@ __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t 
     long long next_check = (long long)a.spill_cycles;
     for (;;) {
         bool want_pop = false;
-        if (kFast && enter && sub && xlen <= kFastM && d0 + d < kFastDepth && row_any(P)) {
+        if (kFast && enter && sub && xlen <= kFastM && row_any(P)) {
             const uint32_t cnt = p <= kFastN ? p : fast_members(P.w[0], X.w[0]);
             if (cnt <= kFastN) {  // this node's whole branch
                 const Row<WPL> R = path_of<WPL>(S + fr0, d, W, Rb);

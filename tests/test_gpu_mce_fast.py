@@ -64,3 +64,23 @@ def test_size_counters_are_emptied_when_full(g2, orc, ctx, monkeypatch, fold):
             c, h = ctx.mce(**kw)
             assert c == want["count"] and int(h.sum()) == c, (fold, kw)
             assert np.array_equal(h, want["hist"][:h.size]), (fold, kw)
+
+
+def test_branches_deep_in_a_root(g2, orc, ctx):
+    """Cliques of 60 to 140 vertices with a few holes each, one of them over a core
+    with many back neighbours: branches enter the register walk at depths from which
+    their sizes exceed its shared counters."""
+    rng = np.random.default_rng(11)
+    edges, base = [], 0
+    for p in (60, 110, 125, 140):
+        a, b = np.triu_indices(p, 1)
+        hole = set(int(x) for x in rng.choice(a.size, 9, replace=False))
+        edges += [(base + int(i), base + int(j)) for t, (i, j) in enumerate(zip(a, b)) if t not in hole]
+        base += p
+    g = g2.Graph.from_edges(base, edges)
+    want = orc.mce(g, threads=8, per_root=True)
+    ctx.load(g)
+    for kw in ({}, {"schedule": "heuristic"}, {"spill_kcycles": 1}, {"flags": 16}):
+        c, h, rn = ctx.mce(root_nodes=True, **kw)
+        assert c == want["count"], kw
+        assert np.array_equal(h, want["hist"][:h.size]) and np.array_equal(rn, want["root_nodes"]), kw
