@@ -84,3 +84,19 @@ def test_branches_deep_in_a_root(g2, orc, ctx):
         c, h, rn = ctx.mce(root_nodes=True, **kw)
         assert c == want["count"], kw
         assert np.array_equal(h, want["hist"][:h.size]) and np.array_equal(rn, want["root_nodes"]), kw
+
+
+def test_levels_above_a_small_branch_are_handed_off(g2, orc, ctx):
+    """A few roots of more than 96 vertices whose depth-1 nodes all enter the register
+    walk: idle warps get the root's own branches, not only those inside a walk."""
+    g = g2.Graph.er(300, 0.4, seed=5).degeneracy_recoded()
+    fwd = np.array([int((g.neighbors(v) > v).sum()) for v in range(g.n)])
+    src = np.flatnonzero(fwd > 96).astype(np.uint32)[-4:]
+    assert src.size == 4
+    want = orc.mce(g, roots=src, threads=8, per_root=True)
+    ctx.load(g)
+    for kw in ({"spill_kcycles": 1}, {}, {"schedule": "heuristic", "spill_kcycles": 1}):
+        c, h, rn = ctx.mce(sources=src, root_nodes=True, **kw)
+        assert c == want["count"] and np.array_equal(h, want["hist"][:h.size]), kw
+        assert np.array_equal(rn, want["root_nodes"]), kw
+        assert ctx.spill_stats()[0] > 200, kw  # the roots were shared out
