@@ -89,7 +89,7 @@ struct MceArgs {
                                          // dropped (set on the device by deadline_set)
     CoreBits core;                  // bit rows (core.bits null: every root takes the general walk)
     uint32_t sorted;                // tasks in descending cost (chunk 0)
-    uint32_t hist_fold;             // a warp's 32-bit size counters are emptied at this count (>= 1)
+    uint32_t hist_fold;             // inner nodes after which a warp empties its 32-bit size counters (a power of two)
 };
 constexpr int kQHead = 0, kQOut = 1;
 constexpr uint32_t kMatchRecordWords = 32;  // stride of a plan-walk record

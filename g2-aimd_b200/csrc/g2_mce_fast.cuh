@@ -82,30 +82,29 @@ __device__ __forceinline__ uint32_t flip32(uint32_t x) {
     return x;
 }
 
-// Counts of cliques of `size` vertices to a 64-bit counter: a root's own (which its
-// commit adds to the run's) or the run's.
-__device__ __forceinline__ void fast_count(const MceArgs &a, unsigned long long *keep, uint32_t size, uint32_t h) {
-    if (keep) keep[size] += h;
-    else if (size < a.hist_len) atomicAdd(a.out + 1 + size, (unsigned long long)h);
-    else if (a.hist_len) atomicOr(a.status, kStatusHistOverflow);  // hist_len 0: no histogram
-}
+// A warp counts clique sizes in 32-bit shared words that live for many walks; word 0
+// (no clique has size 0) carries the inner nodes walked from one walk to the next.
+// An inner node adds at most its kFastN leaves, so emptying the counters at every
+// a.hist_fold-th of them (2^24) keeps each below 2^32.
 
-// The clique sizes a warp has found so far (shared memory) to the run's histogram.
+// To the run's histogram.
 __device__ __noinline__ void fast_flush(const MceArgs &a, uint32_t *hist) {
     __syncwarp();
     for (uint32_t s = lane_id(); s < kFastHist; s += 32) {
         const uint32_t h = hist[s];
         hist[s] = 0;
-        if (h) fast_count(a, nullptr, s, h);
+        if (!h || !s) continue;
+        if (s < a.hist_len) atomicAdd(a.out + 1 + s, (unsigned long long)h);
+        else if (a.hist_len) atomicOr(a.status, kStatusHistOverflow);  // hist_len 0: no histogram
     }
     __syncwarp();
 }
 
-// The same into a root's own counters, which its commit adds to the run's.
+// To a root's own counters, which its commit adds to the run's.
 __device__ __noinline__ void fast_keep(uint32_t *hist, unsigned long long *keep, uint32_t sizes) {
     __syncwarp();
     for (uint32_t s = lane_id(); s < sizes; s += 32) {
-        keep[s] += hist[s];
+        if (s) keep[s] += hist[s];
         hist[s] = 0;
     }
     __syncwarp();
@@ -504,19 +503,16 @@ __device__ __noinline__ FastSum fast_walk(const MceArgs &a, uint32_t task, uint3
         next_check = __shfl_sync(G2_FULL, next_check, 0) / (long long)a.spill_cycles * (long long)a.spill_cycles +
                      (long long)a.spill_cycles;
     }
-    // a maximal clique of `size` vertices; the counters hold 32 bits and live for many
-    // walks, so a full one is emptied on the spot.  Sizes beyond them (a branch deep in
+    uint32_t inner = hist[0];
+    const uint32_t fold = a.hist_fold - 1u;
+    // a maximal clique of `size` vertices.  Sizes beyond the counters (a branch deep in
     // a large root) go to the root's own: keeping such branches out of this walk
     // instead made Chung-Lu 2*10^5 (exponent 2.2) 34 ms where it takes 19
-    const uint32_t full = a.hist_fold;
     auto found = [&](uint32_t size) {
         cliques++;
-        if (lane == 0 && size >= kFastHist) {
-            keep[size]++;
-        } else if (lane == 0) {
-            const uint32_t h = hist[size] + 1u;
-            hist[size] = h == full ? 0u : h;
-            if (h == full) fast_count(a, keep, size, h);
+        if (lane == 0) {
+            if (size < kFastHist) hist[size]++;
+            else keep[size]++;
         }
     };
     auto save = [&](uint32_t at, uint32_t q) {
@@ -576,6 +572,11 @@ __device__ __noinline__ FastSum fast_walk(const MceArgs &a, uint32_t task, uint3
                 const uint32_t step = best >= nb ? N : M;
 #pragma unroll
                 for (int w = 0; w < W; w++) Q[w] = P[w] & ~row[w * step];
+                inner++;
+                if ((inner & fold) == 0) {
+                    if (keep) fast_keep(hist, keep, p + 2u < kFastHist ? p + 2u : kFastHist);
+                    else fast_flush(a, hist);
+                }
                 if (may_spill && (nodes & 15u) == 0) {
                     long long el = 0;
                     if (lane == 0) el = clock64() - c0;
@@ -655,6 +656,7 @@ __device__ __noinline__ FastSum fast_walk(const MceArgs &a, uint32_t task, uint3
         d++;
         enter = true;
     }
+    if (lane == 0) hist[0] = inner;
     __syncwarp();
     return FastSum{nodes, cliques, donated};
 }

@@ -815,14 +815,21 @@ __global__ void __launch_bounds__(256, 3) mce_kernel(const __grid_constant__ Mce
     // (counted once: three atomics on shared words per task cost more than a light root)
     outstanding_add(a, handoff, 1);
     uint32_t chunk = a.chunk ? a.chunk : 1u;
+    const uint32_t nwarps = (uint32_t)(((uint64_t)gridDim.x * blockDim.x) >> 5);
     for (;;) {
         const unsigned long long t0 = grab(a.head, chunk);
         if (t0 >= n) break;
         const unsigned long long t1 = t0 + chunk < n ? t0 + chunk : n;
-        // heavy tasks one at a time, light ones several per atomic: the light end
-        // is the last seven eighths of a cost-ordered list, or the first three
-        // quarters of one in the given (degeneracy) order
-        if (!a.chunk) chunk = a.sorted ? (t0 * 8 > n ? 8u : 1u) : (t0 * 4 < n * 3 ? 4u : 1u);
+        // heavy tasks one at a time; among the light ones (the last seven eighths of a
+        // cost-ordered list, the first three quarters of the vertices in degeneracy
+        // order) several per atomic, as long as four rounds of that many are left for
+        // every warp: a caller's list may hold its heavy roots anywhere, and a short
+        // one would leave most warps without a task
+        if (!a.chunk) {
+            const bool light = a.sorted ? t0 * 8 > n : t0 * 4 < n * 3;
+            const unsigned long long share = (n - t0) / (4ull * nwarps), most = a.sorted ? 8 : 4;
+            chunk = !light || share < 1 ? 1u : (uint32_t)(share < most ? share : most);
+        }
         for (unsigned long long t = t0; t < t1; t++) {
             if (BUDGET && deadline_passed(a)) {  // time budget spent: start no new root
                 if (lane_id() == 0) atomicOr(a.status, kStatusDeadline);

@@ -651,9 +651,9 @@ int mce_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned long
         base.deadline = ctx->d_deadline;
     }
     base.sorted = o && o->schedule != G2_SCHED_GIVEN;
-    base.hist_fold = 1u << 31;
-    if (const char *e = getenv("G2_HIST_FOLD"))  // (tests cross it with few cliques)
-        base.hist_fold = std::max<uint32_t>(1u, (uint32_t)strtoul(e, nullptr, 10));
+    base.hist_fold = 1u << 24;
+    if (const char *e = getenv("G2_HIST_FOLD"))  // (tests cross it with few nodes)
+        base.hist_fold = 1u << std::min<uint32_t>((uint32_t)strtoul(e, nullptr, 10), 24u);
     if (!base.work && !deadline_ms && !tl.split) {  // (those runs take the general walk)
         rc = ensure_clique(ctx, 0, st, &base.core);
         if (rc && rc != G2_ERR_OOM) return rc;

@@ -51,11 +51,11 @@ def test_sources_and_small_slab(g2, orc):
             assert cnt == want["count"] and np.array_equal(h, want["hist"][:h.size]), scratch
 
 
-@pytest.mark.parametrize("fold", [1, 2, 7])
+@pytest.mark.parametrize("fold", [0, 1, 4])
 def test_size_counters_are_emptied_when_full(g2, orc, ctx, monkeypatch, fold):
-    """The warps' 32-bit size counters live for all roots of a warp: with the count at
-    which they are emptied cut to a few cliques, both those of whole roots and those
-    of branches are crossed many times, and the histogram stays the oracle's."""
+    """The warps' 32-bit size counters live for all roots of a warp and are emptied
+    every 2^fold inner nodes: with fold cut from 24 to a few, both those of whole roots
+    and those of branches are emptied many times, and the histogram stays the oracle's."""
     monkeypatch.setenv("G2_HIST_FOLD", str(fold))
     for g in (g2.Graph.rmat(11, 16, seed=2).degeneracy_recoded(), _layers(g2, [97, 130], 0.3, 200, 7)):
         want = orc.mce(g, threads=8)
@@ -100,3 +100,27 @@ def test_levels_above_a_small_branch_are_handed_off(g2, orc, ctx):
         assert c == want["count"] and np.array_equal(h, want["hist"][:h.size]), kw
         assert np.array_equal(rn, want["root_nodes"]), kw
         assert ctx.spill_stats()[0] > 200, kw  # the roots were shared out
+
+
+@pytest.mark.parametrize("take", [1, 5, 600, 5000])
+def test_lists_of_few_roots_are_dealt_out_one_by_one(g2, orc, ctx, take):
+    """The caller's roots, heaviest first, from one to two per resident warp: no warp
+    takes several while others have none, and results follow the caller's order."""
+    g = g2.Graph.er(5000, 0.02, seed=8).degeneracy_recoded()
+    src = np.argsort(-g.degrees(), kind="stable").astype(np.uint32)[:take]
+    want = orc.mce(g, roots=src, threads=8, per_root=True)
+    ctx.load(g)
+    for kw in ({}, {"schedule": "heuristic"}, {"flags": 16}, {"chunk": 3}):
+        c, h, rn = ctx.mce(sources=src, root_nodes=True, **kw)
+        assert c == want["count"] and np.array_equal(h, want["hist"][:h.size]), (take, kw)
+        assert np.array_equal(rn, want["root_nodes"]), (take, kw)
+    if take == 5000:  # one root a grab: no walk waits behind others (a chunk of 8 fills 630 of 3,552 warps)
+        import time
+        def best(**kw):
+            t = []
+            for _ in range(5):
+                t0 = time.perf_counter()
+                ctx.mce(sources=src, **kw)
+                t.append(time.perf_counter() - t0)
+            return min(t)
+        assert best(schedule="heuristic", flags=16) < 1.25 * best(schedule="heuristic", flags=16, chunk=1)
