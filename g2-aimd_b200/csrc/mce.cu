@@ -504,7 +504,7 @@ __device__ int mce_task(const MceArgs &a, uint32_t entry, uint32_t *S, uint32_t 
                 // the levels above it first, whose branches are larger: inside the walk
                 // only its own are handed off, and where every node at depth 1 enters it
                 // a root's warp kept them all (G(500, .3): 4.0 ms, with this 1.5)
-                if (may_spill) {
+                if (may_spill && d > 0) {
                     long long el = 0;
                     if (lane == 0) el = clock64() - c0;
                     el = __shfl_sync(G2_FULL, el, 0);
