@@ -206,12 +206,12 @@ int default_blocks(g2_ctx *ctx, const g2_opts *o, int wpb, int resident_per_sm) 
 }
 
 // Sort the task keys (cost above, slot below).  They are written in slot order
-// and the sort is stable, so the slot bits need no passes: 4 of 8 remain.
-// Costs that are estimates are told apart by their upper 16 bits (sign, exponent
-// and 7 bits: steps of 0.8 %), 2 passes; the caller's scores keep all 32.  (2^20
-// keys: 8 passes 140 us, 2 passes 35 us.)
-int sort_keys(g2_ctx *ctx, uint64_t n, bool estimates, cudaStream_t st) {
-    const int low = estimates ? 48 : 32;
+// and the sort is stable, so the slot bits need no passes: 4 of 8 remain.  (2^20
+// keys: 8 passes 140 us, 4 passes 70 us.  Sorting estimates by their upper 16 bits
+// alone, 2 passes 35 us, made ties of costs up to 0.8 % apart, and with them other
+// roots of a budgeted run finish.)
+int sort_keys(g2_ctx *ctx, uint64_t n, cudaStream_t st) {
+    const int low = 32;
     size_t need = 0;
     cub::DeviceRadixSort::SortKeys(nullptr, need, ctx->d_keys, ctx->d_keys2, (int)n, low, 64, st);
     int rc = cub_space(ctx, need);
@@ -314,7 +314,7 @@ int prepare_tasks(g2_ctx *ctx, const uint32_t *sources, uint64_t nsrc, bool on_d
         // one task per root, descending cost
         cost_keys_kernel<<<ctx->sm_count * 4, 256, 0, st>>>(ctx->d_cost, nsrc, ctx->d_keys);
         ctx->launches++;
-        rc = sort_keys(ctx, nsrc, sched != G2_SCHED_SCORES, st);
+        rc = sort_keys(ctx, nsrc, st);
         if (rc) return rc;
         gather_tasks_kernel<<<ctx->sm_count * 4, 256, 0, st>>>(ctx->d_keys2, roots, nullptr, nsrc, ctx->d_tasks,
                                                               nullptr);
@@ -341,7 +341,7 @@ int prepare_tasks(g2_ctx *ctx, const uint32_t *sources, uint64_t nsrc, bool on_d
                                                            ctx->d_xparts, ctx->d_keys);
     split_total_kernel<<<1, 32, 0, st>>>(S, off, nsrc, cap, ctx->d_ntask);
     ctx->launches += 4;
-    rc = sort_keys(ctx, cap, true, st);
+    rc = sort_keys(ctx, cap, st);
     if (rc) return rc;
     gather_tasks_kernel<<<ctx->sm_count * 4, 256, 0, st>>>(ctx->d_keys2, ctx->d_xroots, ctx->d_xparts, cap,
                                                           ctx->d_tasks, ctx->d_part);

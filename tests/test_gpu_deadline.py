@@ -88,3 +88,23 @@ def test_device_stream_status_reports_the_budget(g2):
             assert code == -11 and int(out[0].item()) < full  # G2_ERR_DEADLINE
         else:
             assert code in (0, -11)
+
+
+def test_budgeted_run_takes_roots_in_exact_cost_order(g2):
+    """One warp under a time budget finishes a prefix of the schedule's order:
+    descending heuristic cost, whole numbers below 2^24 here and many of them within
+    a percent of each other, ties in the caller's order (a shuffled one here)."""
+    from g2aimd.context import Context
+    g = g2.Graph.er(5000, 0.02, seed=8).degeneracy_recoded()
+    d = g.degrees().astype(np.float32)
+    p = np.array([int((g.neighbors(v) > v).sum()) for v in range(g.n)], np.float32)
+    src = np.random.default_rng(2).permutation(g.n).astype(np.uint32)
+    order = np.argsort(-(p * (p + d) + np.float32(1))[src], kind="stable")
+    with Context(0) as c:
+        c.load(g)
+        _n, _h, rn = c.mce(sources=src, root_nodes=True, schedule="heuristic", blocks=1, warps_per_block=1, chunk=1,
+                           deadline_ms=20)
+        assert c.expired
+    done = rn[order] > 0
+    k = int(done.sum())
+    assert 20 < k < g.n and done[:k].all()
