@@ -701,13 +701,9 @@ uint32_t clique_p_fit(uint32_t k, bool in_order, uint64_t words_per_warp, int wa
     return p > kWarpP ? p : kWarpP;
 }
 
-// The limit set on the kernels (not the size of a launch): the same value every
-// time, so that contexts of several threads do not take it from one another.
-constexpr int kMaxDynamic = 200 * 1024;
-
 template <int K, bool O>
 static int clique_occ(int wpb, size_t sm) {
-    cudaFuncSetAttribute(clique_kernel<K, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamic);
+    cudaFuncSetAttribute(clique_kernel<K, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, clique_kernel<K, O>, 32 * wpb, sm) != cudaSuccess) return 0;
     return nb;
@@ -745,7 +741,7 @@ cudaError_t clique_preload() {
 template <int K, bool O>
 static void clique_go(const CliqueArgs &a, int blocks, int wpb, cudaStream_t st) {
     const size_t sm = 4ull * a.smem_words;
-    cudaFuncSetAttribute(clique_kernel<K, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamic);
+    cudaFuncSetAttribute(clique_kernel<K, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     clique_kernel<K, O><<<blocks, 32 * wpb, sm, st>>>(a);
 }
 

@@ -24,6 +24,11 @@ constexpr uint32_t kRecordBit = 0x80000000u;
 // Depth word of a record slot whose reservation ran past the buffer's end.
 constexpr uint32_t kVoidRecord = 0xffffffffu;
 
+// The dynamic shared memory limit set on the kernels (not the size of a launch): the
+// same value every time, so that contexts of several threads do not take it from one
+// another between setting it and launching.
+constexpr int kMaxDynamicSmem = 200 * 1024;
+
 // Bit rows of the last ids of a graph (g2_corebits.cuh): row of vertex u in
 // [base, end) = bits of N+(u) over the ids base, base + 1, ..., `stride` words
 // (a multiple of 4) each, from word `off` of the matrix.  A batch of graphs has

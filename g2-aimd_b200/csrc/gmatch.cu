@@ -968,14 +968,14 @@ size_t match_smem_bytes(int wpl, int warps_per_block, uint32_t p0_words) {
 template <int WPL, bool M, int MINB>
 static void launch_match(const DevPlan &pl, const MatchArgs &a, dim3 g, dim3 b, size_t sm, cudaStream_t st,
                          int cp) {
-    cudaFuncSetAttribute(match_kernel<WPL, M, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(match_kernel<WPL, M, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     match_kernel<WPL, M, MINB><<<g, b, sm, st>>>(a, cp, pl);
 }
 
 template <int WPL, bool M, int MINB>
 static int match_occ(int warps_per_block, uint32_t p0_words) {
     const size_t sm = match_smem_bytes(WPL, warps_per_block, p0_words);
-    cudaFuncSetAttribute(match_kernel<WPL, M, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(match_kernel<WPL, M, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, match_kernel<WPL, M, MINB>, 32 * warps_per_block, sm) !=
         cudaSuccess)

@@ -859,18 +859,18 @@ size_t mce_smem_bytes(int wpl, int warps_per_block) {
 template <int WPL, bool M>
 static void launch_one(const MceArgs &a, dim3 g, dim3 b, size_t sm, cudaStream_t st) {
     if (!M && a.deadline) {  // budgeted runs (never the metrics build)
-        cudaFuncSetAttribute(mce_kernel<WPL, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaFuncSetAttribute(mce_kernel<WPL, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
         mce_kernel<WPL, false, true><<<g, b, sm, st>>>(a);
         return;
     }
-    cudaFuncSetAttribute(mce_kernel<WPL, M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(mce_kernel<WPL, M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     mce_kernel<WPL, M, false><<<g, b, sm, st>>>(a);
 }
 
 template <int WPL, bool M>
 static int mce_occ(int warps_per_block) {
     const size_t sm = mce_smem_bytes(WPL, warps_per_block);
-    cudaFuncSetAttribute(mce_kernel<WPL, M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaFuncSetAttribute(mce_kernel<WPL, M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, mce_kernel<WPL, M, false>, 32 * warps_per_block, sm) !=
         cudaSuccess)
