@@ -298,7 +298,9 @@ __global__ void recode_scatter_kernel(const uint64_t *rp, const uint32_t *ci, co
 
 // Listed rows (distinct ids), renamed and sorted by a bitmap of the new ids in
 // shared memory, a CTA per row and kSpan ids at a time: the cost is the row's
-// entries plus one look at every word of the bitmap, whatever the order.  CUB's
+// entries plus one look at every word of the bitmap, whatever the order.  A row
+// that names a neighbour twice (not a deduplicated list) yields fewer ids than it
+// has entries: *repeated is set and the caller sorts all rows instead.  CUB's
 // segmented sort gives such a row to one CTA for four radix passes over global
 // memory (R-MAT s18: 978 us, and 756 us to scatter the rows a warp each; rows of
 // 1024 entries on here: 85 + 135 us, with 846 us left in the segmented sort).
@@ -309,7 +311,8 @@ constexpr uint64_t kBigVertices = 4ull * kSpan;  // more vertices: too many pass
 __global__ void __launch_bounds__(1024, 1) recode_big_rows_kernel(const uint64_t *rp, const uint32_t *ci,
                                                                   const uint32_t *perm, const uint64_t *new_rp,
                                                                   uint64_t n, const uint32_t *big,
-                                                                  const unsigned long long *nbig, uint32_t *out) {
+                                                                  const unsigned long long *nbig,
+                                                                  unsigned long long *repeated, uint32_t *out) {
     extern __shared__ uint32_t s_map[];
     __shared__ uint32_t s_count[32];
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
@@ -352,6 +355,7 @@ __global__ void __launch_bounds__(1024, 1) recode_big_rows_kernel(const uint64_t
             }
             __syncthreads();  // the bitmap is free again
         }
+        if (threadIdx.x == 0 && base != new_rp[perm[v]] + (hi - lo)) *repeated = 1ull;
     }
 }
 
@@ -461,7 +465,7 @@ cudaError_t recode_device(const uint64_t *rp, const uint32_t *ci, uint64_t n, ui
     max_chunk = std::min<uint64_t>(std::max<uint64_t>(max_chunk, 1), (uint64_t)INT_MAX);
     uint64_t *nrp = nullptr, *deg = nullptr;
     uint32_t *tmp = nullptr, *nci = nullptr, *big = nullptr;
-    unsigned long long *nbig = nullptr;
+    unsigned long long *nbig = nullptr, repeated = 0;  // device: listed rows, and whether one repeats an id
     char *work = nullptr;
     void *scan = nullptr;
     size_t need = 0;
@@ -478,7 +482,7 @@ cudaError_t recode_device(const uint64_t *rp, const uint32_t *ci, uint64_t n, ui
         return o;
     };
     const int G = sms * 8;
-    const uint64_t o_deg = place(8 * (n + 1)), o_tmp = place(4 * std::max<uint64_t>(m, 1)), o_nbig = place(8);
+    const uint64_t o_deg = place(8 * (n + 1)), o_tmp = place(4 * std::max<uint64_t>(m, 1)), o_nbig = place(16);
     // a listed row has at least big_min of the m entries
     const uint64_t o_big = place(4 * (m / big_min + 1));
     if (!ok(cub::DeviceScan::ExclusiveSum(nullptr, need, deg, nrp, (int)(n + 1)))) return e;
@@ -491,7 +495,7 @@ cudaError_t recode_device(const uint64_t *rp, const uint32_t *ci, uint64_t n, ui
     nbig = reinterpret_cast<unsigned long long *>(work + o_nbig);
     big = reinterpret_cast<uint32_t *>(work + o_big);
     scan = work + o_scan;
-    if (!ok(cudaMemsetAsync(deg + n, 0, 8)) || !ok(cudaMemsetAsync(nbig, 0, 8))) goto done;
+    if (!ok(cudaMemsetAsync(deg + n, 0, 8)) || !ok(cudaMemsetAsync(nbig, 0, 16))) goto done;
     recode_degrees_kernel<<<G, 256>>>(rp, perm, n, deg);
     // exclusive scan: row pointers of the renamed rows (entry n = m)
     if (!ok(cub::DeviceScan::ExclusiveSum(scan, need, deg, nrp, (int)(n + 1)))) goto done;
@@ -502,11 +506,15 @@ cudaError_t recode_device(const uint64_t *rp, const uint32_t *ci, uint64_t n, ui
         if (!ok(cudaFuncSetAttribute(recode_big_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      4 * (int)kSpanWords)))
             goto done;
-        recode_big_rows_kernel<<<sms, 1024, sm>>>(rp, ci, perm, nrp, n, big, nbig, nci);
+        recode_big_rows_kernel<<<sms, 1024, sm>>>(rp, ci, perm, nrp, n, big, nbig, nbig + 1, nci);
         if (!ok(cudaGetLastError())) goto done;
     }
     // sort the other rows, in calls of at most max_chunk entries
-    ok(sort_rows_device(nrp, n, m, tmp, nci, max_chunk, sms, big_min));
+    if (!ok(sort_rows_device(nrp, n, m, tmp, nci, max_chunk, sms, big_min))) goto done;
+    if (big_min != ~0ull && m >= big_min && ok(cudaMemcpy(&repeated, nbig + 1, 8, cudaMemcpyDeviceToHost)) && repeated) {
+        recode_scatter_kernel<<<G, 256>>>(rp, ci, perm, nrp, n, ~0ull, big, nbig, tmp);
+        if (ok(cudaGetLastError())) ok(sort_rows_device(nrp, n, m, tmp, nci, max_chunk, sms));
+    }
 done:
     cudaFree(work);
     if (e != cudaSuccess) {
