@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstdint>
+#include <cstdlib>
 #include <vector>
 
 #include "g2_device.cuh"
@@ -49,7 +50,7 @@ constexpr uint32_t kNarrow = 64;          // neighbours of a vertex its claimer 
 constexpr uint32_t kPeelLocal = 24;       // vertices a warp walks from its queue per round
 constexpr uint32_t kPiece = 256;          // neighbours per entry of the shared list
 constexpr uint32_t kNoCore = 0xffffffffu;
-constexpr long long kPeelWait = 1ll << 34;  // longest wait at the grid barrier (SM cycles, ~9 s)
+constexpr long long kPeelWait = 1ll << 37;  // longest wait at the grid barrier (SM cycles, ~70 s)
 
 struct PeelCtl {
     unsigned long long arrived;      // grid barrier: arrivals so far
@@ -68,7 +69,8 @@ __device__ __forceinline__ unsigned long long peel_load(const unsigned long long
 __global__ void __launch_bounds__(kPeelThreads, 1) peel_kernel(const uint64_t *rp, const uint32_t *ci, uint64_t n,
                                                               uint32_t *deg, uint32_t *core, uint32_t *list,
                                                               uint64_t share, uint64_t *shared_list,
-                                                              uint64_t shared_cap, PeelCtl *ctl) {
+                                                              uint64_t shared_cap, PeelCtl *ctl,
+                                                              long long wait_cycles) {
     __shared__ uint32_t s_queue[kPeelWarps][kPeelQueue];
     __shared__ unsigned long long s_claims, s_nshared;
     __shared__ unsigned int s_min, s_bad;
@@ -108,7 +110,7 @@ __global__ void __launch_bounds__(kPeelThreads, 1) peel_kernel(const uint64_t *r
             const long long t0 = clock64();
             s_bad = 0;
             while (peel_load(&ctl->arrived) < want) {
-                if (clock64() - t0 > kPeelWait || *reinterpret_cast<volatile unsigned int *>(&ctl->timeout)) {
+                if (clock64() - t0 > wait_cycles || *reinterpret_cast<volatile unsigned int *>(&ctl->timeout)) {
                     atomicExch(&ctl->timeout, 1u);
                     s_bad = 1;
                     break;
@@ -529,8 +531,8 @@ done:
 
 // perm (new id of each vertex) and core numbers of the CSR (rp, ci) with n
 // vertices; device buffers.  *launches = kernels launched.  Synchronous (the
-// sort's bit count is read back).  cudaErrorLaunchTimeout: the peel's barrier
-// gave up.
+// sort's bit count is read back).  cudaErrorTimeout: the peel's barrier gave up
+// (after kPeelWait, or G2_PEEL_WAIT SM cycles where that is set).
 cudaError_t degeneracy_order_device(const uint64_t *rp, const uint32_t *ci, uint64_t n, uint64_t m, uint32_t *perm,
                                     uint32_t *core, int sms, uint64_t *launches) {
     *launches = 0;
@@ -572,13 +574,15 @@ cudaError_t degeneracy_order_device(const uint64_t *rp, const uint32_t *ci, uint
     uint64_t *shared_list = reinterpret_cast<uint64_t *>(work + o_shared);
     PeelCtl h{};
     int dbits = 0, bits = 0;
-    void *args[] = {&rp, &ci, &n, &deg, &core, &list, &share, &shared_list, &shared_cap, &ctl};
+    long long wait_cycles = kPeelWait;
+    if (const char *env = getenv("G2_PEEL_WAIT")) wait_cycles = strtoll(env, nullptr, 10);
+    void *args[] = {&rp, &ci, &n, &deg, &core, &list, &share, &shared_list, &shared_cap, &ctl, &wait_cycles};
     if (!ok(cudaMemsetAsync(ctl, 0, sizeof(PeelCtl))) ||
         !ok(cudaLaunchCooperativeKernel((const void *)peel_kernel, dim3(blocks), dim3(kPeelThreads), args, 0, nullptr)) ||
         !ok(cudaMemcpy(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost)))
         goto done;
     if (h.timeout) {
-        e = cudaErrorLaunchTimeout;
+        e = cudaErrorTimeout;
         goto done;
     }
     // order by (core, degree, id): a stable sort of the bits that are in use

@@ -32,6 +32,7 @@ namespace g2rt {
 
 int fail_cuda(g2_ctx *c, cudaError_t e, const char *where) {
     if (c) c->cuda_err = std::string(where) + ": " + cudaGetErrorString(e);
+    if (e == cudaErrorTimeout) return G2_ERR_TIMEOUT;  // a kernel's own bounded wait ran out
     return e == cudaErrorMemoryAllocation ? G2_ERR_OOM : G2_ERR_CUDA;
 }
 

@@ -37,3 +37,22 @@ def test_plan_walk_wait_limit_reports_timeout_then_context_recovers(orc, g2):
             c.match(plan, wait_cycles=1, spill_kcycles=1)
         assert err.value.code == G2_ERR_TIMEOUT
         assert c.match(plan) == want
+
+
+@pytest.mark.parametrize("call", ["degeneracy_order", "degeneracy_recode"])
+def test_peel_wait_limit_reports_timeout_then_context_recovers(g2, monkeypatch, call):
+    """The grid barriers of the degeneracy order are bounded too (2^37 cycles; cut to
+    none here): the call reports G2_ERR_TIMEOUT and the context stays usable."""
+    from g2aimd._lib import G2Error
+    from g2aimd.context import Context
+    g = g2.Graph.rmat(12, 12, seed=6)
+    perm_h, core_h = g.degeneracy_order()
+    with Context(0) as c:
+        c.load(g)
+        monkeypatch.setenv("G2_PEEL_WAIT", "-1")
+        with pytest.raises(G2Error) as err:
+            getattr(c, call)()
+        assert err.value.code == G2_ERR_TIMEOUT
+        monkeypatch.delenv("G2_PEEL_WAIT")
+        perm, core = getattr(c, call)()
+        assert np.array_equal(perm, perm_h) and np.array_equal(core, core_h)
