@@ -543,8 +543,9 @@ cudaError_t degeneracy_order_device(const uint64_t *rp, const uint32_t *ci, uint
         return e == cudaSuccess;
     };
     const int G = sms * 8;
-    const unsigned blocks = (unsigned)sms;
-    uint64_t nw = (uint64_t)blocks * kPeelWarps, share = ((n + 31) / 32 + nw - 1) / nw * 32;
+    unsigned blocks = (unsigned)sms;
+    if (const char *env = getenv("G2_PEEL_BLOCKS")) blocks = std::max(1u, std::min(blocks, (unsigned)strtoul(env, nullptr, 10)));
+    uint64_t share = 0;
     uint64_t at = 0;
     auto place = [&](uint64_t bytes) {
         const uint64_t o = at;
@@ -554,7 +555,7 @@ cudaError_t degeneracy_order_device(const uint64_t *rp, const uint32_t *ci, uint
     // peel: degrees, the warps' lists, two shared lists of pieces (each vertex is
     // listed once at most); sort: keys and ids twice
     uint64_t shared_cap = n + m / kPiece;
-    const uint64_t o_ctl = place(sizeof(PeelCtl)), o_deg = place(4 * n), o_list = place(4 * nw * share),
+    const uint64_t o_ctl = place(sizeof(PeelCtl)), o_deg = place(4 * n), o_list = place(4 * (n + 32ull * kPeelWarps * blocks + 64)),
                    o_shared = place(16 * shared_cap), o_keys = place(16 * n), o_ids = place(8 * n);
     size_t need64 = 0, need32 = 0;
     {
@@ -577,9 +578,20 @@ cudaError_t degeneracy_order_device(const uint64_t *rp, const uint32_t *ci, uint
     long long wait_cycles = kPeelWait;
     if (const char *env = getenv("G2_PEEL_WAIT")) wait_cycles = strtoll(env, nullptr, 10);
     void *args[] = {&rp, &ci, &n, &deg, &core, &list, &share, &shared_list, &shared_cap, &ctl, &wait_cycles};
-    if (!ok(cudaMemsetAsync(ctl, 0, sizeof(PeelCtl))) ||
-        !ok(cudaLaunchCooperativeKernel((const void *)peel_kernel, dim3(blocks), dim3(kPeelThreads), args, 0, nullptr)) ||
-        !ok(cudaMemcpy(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost)))
+    if (!ok(cudaMemsetAsync(ctl, 0, sizeof(PeelCtl)))) goto done;
+    // one CTA per SM, or as many as this context may keep resident (part of a GPU)
+    for (;; blocks = (blocks + 1) / 2) {
+        const uint64_t nw = (uint64_t)blocks * kPeelWarps;
+        share = ((n + 31) / 32 + nw - 1) / nw * 32;
+        const cudaError_t r = cudaLaunchCooperativeKernel((const void *)peel_kernel, dim3(blocks), dim3(kPeelThreads), args, 0, nullptr);
+        if (r == cudaErrorCooperativeLaunchTooLarge && blocks > 1) {
+            cudaGetLastError();
+            continue;
+        }
+        if (!ok(r)) goto done;
+        break;
+    }
+    if (!ok(cudaMemcpy(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost)))
         goto done;
     if (h.timeout) {
         e = cudaErrorTimeout;

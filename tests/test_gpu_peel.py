@@ -86,3 +86,16 @@ def test_rows_over_several_spans_of_ids(g2):
         got = c.copy_csr(g.m)
     assert np.array_equal(perm, perm_h) and np.array_equal(core, core_h)
     assert np.array_equal(got.row_ptrs, want.row_ptrs) and np.array_equal(got.cols, want.cols)
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 37])
+def test_order_with_fewer_resident_ctas(g2, monkeypatch, blocks):
+    """A context that may not keep a CTA on every SM peels with fewer."""
+    from g2aimd.context import Context
+    monkeypatch.setenv("G2_PEEL_BLOCKS", str(blocks))
+    g = g2.Graph.rmat(14, 12, seed=4)
+    perm_h, core_h = g.degeneracy_order()
+    with Context(0) as c:
+        c.load(g)
+        perm, core = c.degeneracy_order()
+    assert np.array_equal(core, core_h) and np.array_equal(perm, perm_h)
