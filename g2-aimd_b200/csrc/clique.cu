@@ -269,6 +269,57 @@ __device__ __forceinline__ Root load_root(const CliqueArgs &a, uint32_t task) {
     return r;
 }
 
+// Roots that leave the tiles to the general kernel's forward lists (the rest list).
+// The tiles' cost does not depend on what they hold; the lists' follows the entries
+// (`mean` per head, from 32 heads):
+//  * far: more than a quarter of the heads (8 of a small root) have no bit row.  They
+//    cost a binary search per column, the lists mean / 32 steps and a search each.
+//    G(10^6, 4e-5) 4-cliques 2.4 ms by lists, 2.9 by tiles; G(2*10^5, 10^-3) 7.2 / 13.2.
+//  * Roots of more than 64 vertices with hardly an entry: 4,000 roots over 800 vertices
+//    without an edge, triangles 0.18 / 0.72 ms, 4-cliques 0.69 / 3.5, at a mean of 20
+//    entries 2.8 / 0.72 and 5.5 / 3.5.
+// A warp takes such a root's heads one after the other (0.4 ms for 600), so up to
+// kManySparse of more than 64 vertices in a run stay with the tiles, but for very wide
+// ones (a hub of 20,000 forward neighbours in generator ids: 24 / 102 to 371 ms).
+constexpr uint32_t kFewHeads = 8;
+constexpr uint32_t kSparseP = 64;  // up to here six tiles
+constexpr uint32_t kWideP = 1024;
+constexpr uint32_t kManySparse = 1024;
+__device__ __forceinline__ bool heads_far(const CliqueArgs &a, const CoreBlock &b, uint64_t ids, uint64_t p) {
+    return p > kFewHeads && ldg(a.ci + ids + (p <= 32u ? kFewHeads : p / 4u)) < b.base;
+}
+__device__ __forceinline__ uint32_t forward_length(const CliqueArgs &a, uint32_t u) {
+    const uint64_t len = ldg(a.rp + u + 1) - ldg(a.rp + u) - ldg(a.fo + u);
+    return (uint32_t)(len < (1u << 26) ? len : 1u << 26);
+}
+// A root of up to kSparseP vertices, per lane (from 4 heads).
+__device__ __forceinline__ bool small_leaves_tiles(const CliqueArgs &a, const CoreBlock &b, uint64_t ids, uint64_t p) {
+    if (!heads_far(a, b, ids, p)) return false;
+    uint64_t sum = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) sum += forward_length(a, ldg(a.ci + ids + p * (2 * i + 1) / 8u));
+    return sum / 4u + 32u < 3u * p;
+}
+// A wider one (one warp).
+__device__ __forceinline__ bool wide_leaves_tiles(const CliqueArgs &a, uint32_t k, const CoreBlock &b, uint64_t ids,
+                                                  uint64_t p) {
+    const uint32_t len = forward_length(a, ldg(a.ci + ids + p * lane_id() / 32u));
+    const uint64_t mean = __reduce_add_sync(G2_FULL, len) / 32u;
+    return mean * (k == 3 ? 128u : k == 4 ? 64u : 16u) < p || (mean + 32u < 3u * p && heads_far(a, b, ids, p));
+}
+// Does root r leave the tiles?  many: the run holds many such roots.  Warp-uniform.
+__device__ __forceinline__ bool leaves_tiles(const CliqueArgs &a, uint32_t k, const CoreBlock &b, const Root &r,
+                                             bool many) {
+    if (r.p <= (many ? kSparseP : kWideP) || !a.by_cost) return false;  // (small ones: by the preparation)
+    return wide_leaves_tiles(a, k, b, r.ids, r.p);
+}
+__device__ __forceinline__ bool many_sparse(const CliqueArgs &a) { return a.by_cost && a.counts[5] > kManySparse; }
+
+// A root to the rest list (one lane).
+__device__ __forceinline__ void to_rest(const CliqueArgs &a, uint32_t task) {
+    a.lists[3 * a.list_cap + atomicAdd(a.counts + 3, 1ull)] = task;
+}
+
 // p <= 32: lane j holds P0[j] and its row.  Warp total.
 template <int K>
 __device__ uint64_t root_small(const Csr &g, const CoreBlock &b, const Root &r, uint32_t id) {
@@ -383,7 +434,7 @@ __device__ __forceinline__ Sub make_sub(uint32_t *at, uint32_t cap) {
 // One warp takes root r.  area: the warp's shared memory (P0, rows, 5-clique work).
 template <int K, bool ORDER>
 __device__ __forceinline__ void warp_task(const CliqueArgs &a, const Csr &g, const Root &r, uint32_t id,
-                                          uint32_t *area, uint32_t *slab, uint64_t &total) {
+                                          uint32_t *area, uint32_t *slab, bool many, uint64_t &total) {
     long long c0 = 0;
     if (a.root_cost) c0 = clock64();
     uint32_t *p0s = area, *A = area + kWarpP;
@@ -393,6 +444,9 @@ __device__ __forceinline__ void warp_task(const CliqueArgs &a, const Csr &g, con
     uint64_t c = 0;
     if (past_deadline(a)) {
         c = ~0ull;
+    } else if (leaves_tiles(a, K, b, r, many)) {
+        if (lane == 0) to_rest(a, r.task);
+        return;
     } else if (r.p <= 32u) {
         c = root_small<K>(g, b, r, id);
     } else if (r.p <= kWarpP) {
@@ -416,7 +470,7 @@ __device__ __forceinline__ void warp_task(const CliqueArgs &a, const Csr &g, con
 // (and the first 32 ids of P0 of the next one) ahead of the walk.
 template <int K, bool ORDER>
 __device__ __forceinline__ void warp_list(const CliqueArgs &a, const Csr &g, uint32_t list, uint32_t chunk,
-                                          uint32_t *area, uint32_t *slab, uint64_t &total) {
+                                          uint32_t *area, uint32_t *slab, bool many, uint64_t &total) {
     const uint32_t lane = lane_id();
     const uint32_t *ids = a.lists + (uint64_t)list * a.list_cap;
     const uint64_t n = a.counts[list];
@@ -443,15 +497,15 @@ __device__ __forceinline__ void warp_list(const CliqueArgs &a, const Csr &g, uin
             r.ids = __shfl_sync(G2_FULL, mine.ids, t);
             const uint32_t id = next;
             if (t + 1 < m) fetch(t + 1);
-            warp_task<K, ORDER>(a, g, r, id, area, slab, total);
+            warp_task<K, ORDER>(a, g, r, id, area, slab, many, total);
         }
     }
 }
 
 // The CTA's warps share each root of list 0.
 template <int K>
-__device__ __forceinline__ uint64_t cta_list(const CliqueArgs &a, const Csr &g, uint32_t *smem) {
-    __shared__ uint32_t s_entry, s_next, s_expired, s_late;
+__device__ __forceinline__ uint64_t cta_list(const CliqueArgs &a, const Csr &g, uint32_t *smem, bool many) {
+    __shared__ uint32_t s_entry, s_next, s_expired, s_late, s_rest;
     __shared__ unsigned long long s_count;
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
     uint32_t *slab = a.scratch + (uint64_t)blockIdx.x * nw * a.words_per_warp;
@@ -475,8 +529,10 @@ __device__ __forceinline__ uint64_t cta_list(const CliqueArgs &a, const Csr &g, 
         const uint32_t entry = s_entry;
         if (entry == 0xffffffffu) break;
         Root r = load_root(a, a.lists[entry]);
+        bool first = true;  // of the root's pieces
         if (K == 5 && a.pieces) {  // piece of a heavy root
             const uint32_t piece = a.pieces[entry];
+            first = (piece & 0xffffu) == 0;
             r.part += r.nparts * (piece & 0xffffu);
             r.nparts *= piece >> 16;
         }
@@ -487,7 +543,15 @@ __device__ __forceinline__ uint64_t cta_list(const CliqueArgs &a, const Csr &g, 
         const bool staged = r.p <= room_words;
         if (staged)
             for (uint32_t i = threadIdx.x; i < r.p; i += blockDim.x) room[i] = ldg(a.ci + r.ids + i);
+        if (wib == nw - 1) {  // (while the others still load)
+            const bool rest = !s_late && leaves_tiles(a, K, b, r, many);
+            if (lane == 0) {
+                s_rest = rest;  // (read by all before the next iteration's first barrier, written after it)
+                if (rest && first) to_rest(a, r.task);
+            }
+        }
         __syncthreads();
+        if (s_rest) continue;
         uint64_t c = 0;
         if (!s_late) {  // (else the time budget is spent: start no new root)
             if constexpr (K == 3) {
@@ -543,21 +607,22 @@ __global__ void __launch_bounds__(256, K == 5 ? 4 : 5) clique_kernel(const __gri
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const Csr g{a.rp, a.ci, a.fo, a.core.bits};
     uint64_t total = 0;
-    if (!ORDER) total = cta_list<K>(a, g, smem);
+    const bool many = many_sparse(a);
+    if (!ORDER) total = cta_list<K>(a, g, smem, many);
     uint32_t *area = smem + wib * warp_area(K, ORDER, a.q_words);
     uint32_t *slab = a.scratch + ((uint64_t)blockIdx.x * nw + wib) * a.words_per_warp;
     uint64_t mine = 0;
     if (ORDER) {
-        warp_list<K, true>(a, g, 0, a.chunk, area, slab, mine);
+        warp_list<K, true>(a, g, 0, a.chunk, area, slab, many, mine);
     } else {
-        warp_list<K, false>(a, g, 1, 1u, area, slab, mine);
-        warp_list<K, false>(a, g, 2, 8u, area, slab, mine);
+        warp_list<K, false>(a, g, 1, 1u, area, slab, many, mine);
+        warp_list<K, false>(a, g, 2, 8u, area, slab, many, mine);
     }
     if (lane == 0) total += mine;
     if (lane == 0 && total) atomicAdd(a.out, (unsigned long long)total);
 }
 
-// Cube of |P0| per CTA piece of a 5-clique root (p = 101).
+// |P0| times the square of its vertices' neighbourhoods per CTA piece of a 5-clique root.
 constexpr uint64_t kPieceCube = 1ull << 20;
 
 // Segment of a bit row kept in a warp's shared memory while it is filled (words).
@@ -625,19 +690,51 @@ __global__ void __launch_bounds__(256) clique_prepare_kernel(const __grid_consta
         const uint64_t t = t0 + lane;
         int list = -1;
         uint32_t copies = 1;
+        uint32_t v = 0;
+        uint64_t ids = 0, p = 0;
         if (t < nt) {
-            const uint32_t v = a.tasks[t];
-            const uint64_t p = ldg(a.rp + v + 1) - ldg(a.rp + v) - ldg(a.fo + v);
+            v = a.tasks[t];
+            ids = ldg(a.rp + v) + ldg(a.fo + v);
+            p = ldg(a.rp + v + 1) - ids;
+        }
+        bool sparse = false;
+        if (a.by_cost) {
+            const CoreBlock b = core_block(a.core, v);
+            if (p + 1 >= k && p <= kSparseP) sparse = small_leaves_tiles(a, b, ids, p);
+            // how many wider roots leave the tiles: the first of the 32 stands for all
+            const uint32_t m = __ballot_sync(G2_FULL, p > kSparseP && p <= a.p_fit), l = m ? __ffs(m) - 1 : 0;
+            const uint32_t lv = __shfl_sync(G2_FULL, v, l);
+            if (m && wide_leaves_tiles(a, k, core_block(a.core, lv), __shfl_sync(G2_FULL, ids, l),
+                                       __shfl_sync(G2_FULL, p, l)) && lane == 0)
+                atomicAdd(a.counts + 5, (unsigned long long)__popc(m));
+        }
+        // share of the pairs in P0 that are edges, of 32 (5-cliques of wide roots, for their pieces)
+        uint32_t share = 32;
+        if (a.pieces && !a.in_order) {
+            const bool look = p > a.cta_min && p <= a.p_fit && p * p * p > kPieceCube;
+            for (uint32_t m = __ballot_sync(G2_FULL, look); m; m &= m - 1) {
+                const uint32_t l = __ffs(m) - 1;
+                const uint64_t half = __shfl_sync(G2_FULL, p, l) / 2u, at = __shfl_sync(G2_FULL, ids, l);
+                const uint32_t u = ldg(a.ci + at + half * lane / 32u);
+                const uint32_t y = ldg(a.ci + at + half + half * ((7u * lane + 3u) & 31u) / 32u);
+                const bool hit = contains(a.ci, ldg(a.rp + u) + ldg(a.fo + u), ldg(a.rp + u + 1), y);
+                const uint32_t hits = __popc(__ballot_sync(G2_FULL, hit));
+                if (l == lane) share = hits ? hits : 1u;
+            }
+        }
+        if (t < nt) {
             if (p + 1 < k) {  // no k-clique rooted here: finished
                 if (a.root_cost) a.root_cost[t] = 1;
-            } else if (p > a.p_fit) {
+            } else if (p > a.p_fit || sparse) {
                 list = 3;
             } else {
                 list = a.in_order ? 0 : p > a.cta_min ? 0 : p > 32u ? 1 : 2;
-                // 5-cliques of a wide root cost about p^3: pieces of about
-                // kPieceCube, each a CTA's share of the highest vertices
-                if (a.pieces && list == 0 && !a.in_order && p * p * p > kPieceCube) {
-                    const uint64_t want = p * p * p / kPieceCube + 1;
+                // 5-cliques of a wide root cost about p times the square of its
+                // vertices' neighbourhoods: pieces of about kPieceCube, each a CTA's
+                // share of the highest vertices
+                const uint64_t in = p * share / 32u;
+                if (a.pieces && list == 0 && !a.in_order && p * in * in > kPieceCube) {
+                    const uint64_t want = p * in * in / kPieceCube + 1;
                     copies = (uint32_t)(want < 64 ? want : 64);
                     if (atomicAdd(a.counts + 4, copies - 1ull) + copies - 1 > a.extra_cap) copies = 1;
                 }
@@ -690,9 +787,10 @@ uint32_t clique_smem_words(uint32_t k, bool in_order, uint32_t max_fwd, int warp
     return words;
 }
 
-uint32_t clique_p_fit(uint32_t k, bool in_order, uint64_t words_per_warp, int warps_per_block, uint32_t smem_words) {
-    (void)smem_words;
-    if (k == 3) return 0xffffffffu;
+bool clique_by_cost(uint32_t max_fwd, bool whole) { return !whole || max_fwd > kSparseP; }
+
+uint32_t clique_p_fit(uint32_t k, bool in_order, uint64_t words_per_warp, int warps_per_block) {
+    if (k == 3) return 1u << 18;  // (a lane counts a root's edges in 32 bits)
     uint64_t words = in_order ? words_per_warp : words_per_warp * (uint64_t)warps_per_block;
     uint32_t W = 0;
     const uint32_t wmax = k == 5 ? kMaxQWords : 4096u;

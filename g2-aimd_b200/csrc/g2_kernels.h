@@ -201,10 +201,11 @@ struct CliqueArgs {
     uint32_t in_order;              // one list in task order (else lists by root size)
     uint32_t cta_min;               // lists by size: roots with larger |P0| are shared by a CTA
     uint32_t p_fit;                 // roots with larger |P0| go to the rest list
+    uint32_t by_cost;               // so do those whose forward lists are cheaper than their tiles
     uint32_t *lists;                // four lists of list_cap task ids: by size (or [0] in order), [3] rest
     uint32_t *pieces;               // 5-cliques, lists by size: (pieces << 16) | piece of list 0's entries
     uint64_t list_cap, extra_cap;   // list_cap >= ntasks + extra_cap; extra_cap = pieces beyond one per root
-    unsigned long long *counts;     // list lengths; [4] extra pieces
+    unsigned long long *counts;     // list lengths; [4] extra pieces, [5] roots whose lists are cheaper (about)
     unsigned long long *heads;      // list heads
     uint32_t chunk;                 // in-order runs: tasks per queue atomic
     uint32_t *scratch;              // per-warp slabs
@@ -220,7 +221,9 @@ struct CliqueArgs {
 // Largest |P0| that one warp walks in runs by size.
 uint32_t clique_cta_min(uint32_t k);
 // Largest |P0| a launch of this geometry counts itself.
-uint32_t clique_p_fit(uint32_t k, bool in_order, uint64_t words_per_warp, int warps_per_block, uint32_t smem_words);
+uint32_t clique_p_fit(uint32_t k, bool in_order, uint64_t words_per_warp, int warps_per_block);
+// Can a root's forward lists be cheaper than its tiles?  (whole: every id has a bit row)
+bool clique_by_cost(uint32_t max_fwd, bool whole);
 // Dynamic shared memory (words) for roots up to max_fwd, and a row's word count for 5-cliques.
 uint32_t clique_smem_words(uint32_t k, bool in_order, uint32_t max_fwd, int warps_per_block, uint32_t *q_words);
 int clique_blocks_per_sm(uint32_t k, bool in_order, int warps_per_block, uint32_t smem_words);

@@ -229,6 +229,8 @@ bool clique_run(const g2_ctx *ctx, const g2_opts *o) {
            !(o && (o->flags & G2_FLAG_WORK_MODEL));
 }
 
+constexpr uint32_t kSplitForward = 2048;  // clique runs with wider roots split the heavy ones
+
 // Task generation: upload the roots, compute the schedule's cost per root (the
 // learned model's features + MLP run here, in one kernel), optionally split
 // heavy roots, sort the tasks by descending cost.  No host synchronisation.
@@ -246,9 +248,11 @@ int prepare_tasks(g2_ctx *ctx, const uint32_t *sources, uint64_t nsrc, bool on_d
     if (sched == G2_SCHED_LEARNED && !ctx->d_model) return G2_ERR_INVALID;
     // MCE balances inside roots by handing branches to idle warps, and 3- to
     // 5-clique runs by sharing a root's rows among a CTA's warps, which split
-    // tasks cannot do: there the static split is only taken when asked for
+    // tasks cannot do: there the static split is only taken when asked for (or when
+    // roots may be so wide that a warp walks their lists: hubs in generator ids)
+    const bool shared = clique_run(ctx, o) && ctx->max_fwd <= kSplitForward;
     const bool split = nsrc > 0 && (sched == G2_SCHED_HEURISTIC || sched == G2_SCHED_LEARNED) &&
-                       ((flags & G2_FLAG_SPLIT) || (!mce && !clique_run(ctx, o) && sched == G2_SCHED_LEARNED &&
+                       ((flags & G2_FLAG_SPLIT) || (!mce && !shared && sched == G2_SCHED_LEARNED &&
                                                     !(flags & G2_FLAG_NO_SPLIT)));
     // sum_i ceil(c_i / t) <= n + total / t = n + g * warps
     const uint32_t gran = (o && o->split_granularity) ? std::min<uint32_t>(o->split_granularity, 1024u) : 4u;
@@ -368,7 +372,7 @@ int ensure_scratch(g2_ctx *ctx) {
 // Device counters: queue heads of the passes, deferred-list sizes, hand-off
 // record / pool allocation and the record queue.
 constexpr int kCtrHead = 0;    // 3 queue heads
-constexpr int kCtrClique = 4;  // clique runs: 4 list lengths, extra pieces, then 3 list heads
+constexpr int kCtrClique = 4;  // clique runs: 4 list lengths, extra pieces, sparse roots, then 3 list heads
 constexpr int kCtrDefer = 16;  // 3 deferred-list sizes
 constexpr int kCtrRec = 19;    // records reserved
 constexpr int kCtrPool = 20;   // pool units (64 words) used
@@ -918,14 +922,15 @@ int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned lo
         // a budgeted run drops an unfinished root whole: no pieces
         if (ctx->plan.k == 5 && !a.deadline) q.pieces = ctx->d_clists + 4 * q.list_cap;
         q.counts = ctx->d_ctr + kCtrClique;
-        q.heads = ctx->d_ctr + kCtrClique + 5;
+        q.heads = ctx->d_ctr + kCtrClique + 6;
         q.chunk = std::min<uint32_t>((o && o->chunk) ? o->chunk : 1u, 32u);
         q.scratch = ctx->d_scratch;
         q.words_per_warp = (ctx->scratch_words / ((uint64_t)cg.blocks * cg.wpb)) & ~63ull;
         q.smem_words = cg.smem_words;
         q.q_words = cg.q_words;
         q.cta_min = g2::clique_cta_min(ctx->plan.k);
-        q.p_fit = g2::clique_p_fit(ctx->plan.k, cg.in_order, q.words_per_warp, cg.wpb, cg.smem_words);
+        q.p_fit = g2::clique_p_fit(ctx->plan.k, cg.in_order, q.words_per_warp, cg.wpb);
+        q.by_cost = g2::clique_by_cost(ctx->max_fwd, q.core.rows == ctx->n);
         q.out = d_out;
         q.root_nodes = d_root_nodes;
         q.root_cost = d_root_cost;
@@ -946,11 +951,11 @@ int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned lo
         if (e == cudaSuccess) e = g2::clique_launch(q, ctx->plan.k, cg.blocks, cg.wpb, st);
         if (e != cudaSuccess) return fail_cuda(ctx, e, "clique_launch");
         ctx->launches += 2;
-        // roots wider than the rows' room, counted by the general kernel
+        // roots wider than the rows' room or cheaper by their lists, counted by the general kernel
         a.task_index = q.lists + 3 * q.list_cap;
         a.ntasks_dev = q.counts + 3;
     }
-    if (!rows || ctx->max_fwd > q.p_fit) {
+    if (!rows || q.by_cost || ctx->max_fwd > q.p_fit) {
         e = g2::match_launch(ctx->plan, a, blocks, wpb, st, clique, wpl, o ? (int)o->ctas_per_sm : 0);
         ctx->launches++;
     }

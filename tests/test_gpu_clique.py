@@ -88,3 +88,65 @@ def test_batch_blocks(g2, orc, ctx):
         want = [orc.match(g, plan, threads=4)["count"] if g.n else 0 for g in gs]
         for kw in ({}, {"schedule": "heuristic"}):
             assert ctx.batch_match(plan, **kw).tolist() == want, (q, kw)
+
+
+def _csr(g2, n, e):
+    e = np.asarray(e, np.int64)
+    e = e[e[:, 0] != e[:, 1]]
+    key = np.unique(np.concatenate([e[:, 0] * n + e[:, 1], e[:, 1] * n + e[:, 0]]))
+    rp = np.zeros(n + 1, np.uint64)
+    rp[1:] = np.cumsum(np.bincount(key // n, minlength=n))
+    return g2.Graph(rp, (key % n).astype(np.uint32))
+
+
+def _sparse(g2, which):
+    """Graphs whose roots are cheaper by their forward lists than by tiles."""
+    rng = np.random.default_rng(4)
+    if which == "far":  # small roots whose heads have no bit row
+        return _csr(g2, 60000, np.stack([rng.integers(0, 60000, 900000), rng.integers(0, 60000, 900000)], 1))
+    if which == "many":  # 1,300 roots of 65 to 300 vertices with hardly an edge among them
+        d = np.tile([65, 66, 100, 129, 300], 260)
+        e = np.stack([np.repeat(np.arange(1300), d), 1300 + rng.integers(0, 600, d.sum())], 1)
+        return _csr(g2, 1900, np.concatenate([e, np.stack([1300 + rng.integers(0, 600, 500),
+                                                           1300 + rng.integers(0, 600, 500)], 1)]))
+    hub = np.stack([np.zeros(11999, int), np.arange(1, 12000)], 1)  # one wide root, a few triangles
+    return _csr(g2, 12000, np.concatenate([hub, rng.integers(1, 12000, (3000, 2))]))
+
+
+@pytest.mark.parametrize("which", ["far", "many", "hub"])
+@pytest.mark.parametrize("q", [0, 24, 25])
+def test_sparse_roots_by_their_lists(g2, orc, ctx, q, which):
+    from g2aimd.context import Plan
+    plan = Plan.preset(q)
+    g = _sparse(g2, which)
+    want = orc.match(g, plan, threads=8, per_root=True)
+    src = np.arange(g.n - 1, -1, -3, dtype=np.uint32)
+    ctx.load(g)
+    for kw in ({}, {"schedule": "heuristic"}, {"schedule": "heuristic", "split": True, "granularity": 64},
+               {"chunk": 5, "warps_per_block": 2}, {"schedule": "heuristic", "deadline_ms": 600000}):
+        rc = np.zeros(g.n, np.uint64)
+        assert ctx.match(plan, root_counts=rc, **kw) == want["count"], kw
+        assert np.array_equal(rc, want["root_counts"]), kw
+        assert ctx.match(plan, sources=src, **kw) == int(want["root_counts"][src].sum()), kw
+
+
+@pytest.mark.parametrize("q,which", [(0, "hub"), (24, "many"), (25, "many")])
+def test_sparse_roots_cost_what_they_hold(g2, ctx, q, which):
+    """Roots with next to no cliques: the many take no longer than three plan walks, the
+    hub (whose dense tiles took one warp 130 ms) no longer than 60 ms."""
+    import time
+    from g2aimd.context import Plan
+    plan = Plan.preset(q)
+    ctx.load(_sparse(g2, which))
+
+    def best(**kw):
+        t = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            ctx.match(plan, **kw)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    for schedule in ("given", "heuristic"):
+        limit = 0.06 if which == "hub" else 3 * best(schedule=schedule, intersect_mode=1)
+        assert best(schedule=schedule) < limit, schedule
