@@ -72,6 +72,8 @@ struct Tri {
     }
 };
 
+// Checks inside a root's tiles stand in the BUDGET build only (deadline set): in the
+// other they cost 4 % of the 4-cliques of R-MAT s20.
 __device__ __forceinline__ bool past_deadline(const CliqueArgs &a) {
     if (!a.deadline) return false;
     unsigned long long now = 0;
@@ -150,11 +152,16 @@ __device__ __forceinline__ uint32_t tile_chunk(const Tri &t, uint32_t p, uint32_
     return pair_chunk_n(t, p, w, j0, j1 - j0, part, nparts);
 }
 
-// Triangles of a local graph of p vertices, by one warp.  Per-lane count.
-__device__ __forceinline__ uint64_t triangles(const Tri &t, uint32_t p, uint32_t part, uint32_t nparts) {
+// Triangles of a local graph of p vertices, by one warp.  Per-lane count; ~0 if the
+// time budget of `budget` ran out.
+template <bool BUDGET>
+__device__ __forceinline__ uint64_t triangles(const Tri &t, uint32_t p, uint32_t part, uint32_t nparts,
+                                              const CliqueArgs *budget = nullptr) {
     uint64_t c = 0;
-    for (uint32_t w = 0; 32u * w < p; w++)
+    for (uint32_t w = 0; 32u * w < p; w++) {
+        if (BUDGET && past_deadline(*budget)) return ~0ull;
         for (uint32_t k = 0; k < chunks_of(w); k++) c += tile_chunk(t, p, w, k, part, nparts);
+    }
     return c;
 }
 
@@ -208,7 +215,7 @@ __device__ uint64_t count_below(const Tri &t, uint32_t top, const Sub &sub) {
             if (done < c0 + 32u && (done & 31u)) row[done >> 5] = acc >> (32u - (done & 31u));
         }
         __syncwarp();
-        const uint64_t c = triangles(s, q, 0u, 1u);
+        const uint64_t c = triangles<false>(s, q, 0u, 1u);
         __syncwarp();  // the list and rows are free again
         return c;
     }
@@ -347,13 +354,15 @@ __device__ uint64_t root_small(const Csr &g, const CoreBlock &b, const Root &r, 
     return __reduce_add_sync(G2_FULL, n);
 }
 
-// Triangles of root r: edges of its local graph, by tiles k = first, first + step, ...  Per-lane count.
-template <class P0>
-__device__ __forceinline__ uint64_t count_edges(const Csr &g, const CoreBlock &b, P0 ids, const Root &r,
+// Triangles of root r: edges of its local graph, by tiles k = first, first + step, ...
+// Per-lane count; ~0 if the time budget ran out (looked at once per row of tiles).
+template <bool BUDGET, class P0>
+__device__ __forceinline__ uint64_t count_edges(const CliqueArgs &a, const Csr &g, const CoreBlock &b, P0 ids, const Root &r,
                                                 uint32_t first, uint32_t step) {
     const uint32_t lane = lane_id();
     uint32_t c = 0, k = 0;
     for (uint32_t w = 0; 32u * w < r.p; w++) {
+        if (BUDGET && past_deadline(a)) return ~0ull;
         const bool mine = r.nparts <= 1 || (32u * w + lane) % r.nparts == r.part;
         for (uint32_t q = 0; q <= w; q++, k++) {
             if (k % step != first) continue;
@@ -364,29 +373,36 @@ __device__ __forceinline__ uint64_t count_edges(const Csr &g, const CoreBlock &b
     return c;
 }
 
-// Rows of root r into t, by tiles k = first, first + step, ...
-template <class P0>
-__device__ __forceinline__ void build_rows(const Csr &g, const CoreBlock &b, P0 ids, uint32_t p, const Tri &t,
+// Rows of root r into t, by tiles k = first, first + step, ...  false if the time
+// budget ran out (looked at once per row of tiles).
+template <bool BUDGET, class P0>
+__device__ __forceinline__ bool build_rows(const CliqueArgs &a, const Csr &g, const CoreBlock &b, P0 ids, uint32_t p, const Tri &t,
                                            uint32_t first, uint32_t step) {
     uint32_t k = 0;
     for (uint32_t w = 0; 32u * w < p; w++) {
+        if (BUDGET && past_deadline(a)) return false;
         uint32_t *row = t.row(32u * w + lane_id());
         for (uint32_t q = 0; q <= w; q++, k++)
             if (k % step == first) row[q] = local_word(g, b, ids, p, w, q);
     }
+    return true;
 }
 
 // One warp: rows in `A`, P0 at `ids`.  Warp total; ~0 if the time budget ran out.
-template <int K, class P0>
+template <int K, bool BUDGET, class P0>
 __device__ __forceinline__ uint64_t root_warp(const CliqueArgs &a, const Csr &g, const CoreBlock &b, const Root &r,
                                               P0 ids, uint32_t *A, const Sub &sub) {
-    if constexpr (K == 3) return warp_sum_u64(count_edges(g, b, ids, r, 0u, 1u));
+    if constexpr (K == 3) {
+        const uint64_t n = count_edges<BUDGET>(a, g, b, ids, r, 0u, 1u);
+        return BUDGET && n == ~0ull ? n : warp_sum_u64(n);
+    }
     const Tri t{A};
-    build_rows(g, b, ids, r.p, t, 0u, 1u);
+    if (!build_rows<BUDGET>(a, g, b, ids, r.p, t, 0u, 1u) && BUDGET) return ~0ull;
     __syncwarp();
     uint64_t c = 0;
     if constexpr (K == 4) {
-        c = triangles(t, r.p, r.part, r.nparts);
+        c = triangles<BUDGET>(t, r.p, r.part, r.nparts, &a);
+        if (BUDGET && c == ~0ull) return c;
     } else {
         for (uint32_t x = 3; x < r.p; x++) {
             if (r.nparts > 1 && x % r.nparts != r.part) continue;
@@ -432,7 +448,7 @@ __device__ __forceinline__ Sub make_sub(uint32_t *at, uint32_t cap) {
 }
 
 // One warp takes root r.  area: the warp's shared memory (P0, rows, 5-clique work).
-template <int K, bool ORDER>
+template <int K, bool ORDER, bool BUDGET>
 __device__ __forceinline__ void warp_task(const CliqueArgs &a, const Csr &g, const Root &r, uint32_t id,
                                           uint32_t *area, uint32_t *slab, bool many, uint64_t &total) {
     long long c0 = 0;
@@ -453,10 +469,10 @@ __device__ __forceinline__ void warp_task(const CliqueArgs &a, const Csr &g, con
         p0s[lane] = id;
         for (uint32_t i = 32u + lane; i < r.p; i += 32) p0s[i] = ldg(a.ci + r.ids + i);
         __syncwarp();
-        c = root_warp<K>(a, g, b, r, (const uint32_t *)p0s, A, sub);
+        c = root_warp<K, BUDGET>(a, g, b, r, (const uint32_t *)p0s, A, sub);
         __syncwarp();
     } else if (ORDER) {
-        c = root_warp<K>(a, g, b, r, a.ci + r.ids, slab, sub);
+        c = root_warp<K, BUDGET>(a, g, b, r, a.ci + r.ids, slab, sub);
     }
     if (c == ~0ull) {
         if (lane == 0) atomicOr(a.status, kStatusDeadline);
@@ -468,7 +484,7 @@ __device__ __forceinline__ void warp_task(const CliqueArgs &a, const Csr &g, con
 
 // Warps take runs of `chunk` tasks of a list; the lanes read the tasks' roots
 // (and the first 32 ids of P0 of the next one) ahead of the walk.
-template <int K, bool ORDER>
+template <int K, bool ORDER, bool BUDGET>
 __device__ __forceinline__ void warp_list(const CliqueArgs &a, const Csr &g, uint32_t list, uint32_t chunk,
                                           uint32_t *area, uint32_t *slab, bool many, uint64_t &total) {
     const uint32_t lane = lane_id();
@@ -497,13 +513,13 @@ __device__ __forceinline__ void warp_list(const CliqueArgs &a, const Csr &g, uin
             r.ids = __shfl_sync(G2_FULL, mine.ids, t);
             const uint32_t id = next;
             if (t + 1 < m) fetch(t + 1);
-            warp_task<K, ORDER>(a, g, r, id, area, slab, many, total);
+            warp_task<K, ORDER, BUDGET>(a, g, r, id, area, slab, many, total);
         }
     }
 }
 
 // The CTA's warps share each root of list 0.
-template <int K>
+template <int K, bool BUDGET>
 __device__ __forceinline__ uint64_t cta_list(const CliqueArgs &a, const Csr &g, uint32_t *smem, bool many) {
     __shared__ uint32_t s_entry, s_next, s_expired, s_late, s_rest;
     __shared__ unsigned long long s_count;
@@ -555,13 +571,18 @@ __device__ __forceinline__ uint64_t cta_list(const CliqueArgs &a, const Csr &g, 
         uint64_t c = 0;
         if (!s_late) {  // (else the time budget is spent: start no new root)
             if constexpr (K == 3) {
-                if (staged) c = count_edges(g, b, (const uint32_t *)room, r, wib, nw);
-                else c = count_edges(g, b, a.ci + r.ids, r, wib, nw);
+                if (staged) c = count_edges<BUDGET>(a, g, b, (const uint32_t *)room, r, wib, nw);
+                else c = count_edges<BUDGET>(a, g, b, a.ci + r.ids, r, wib, nw);
+                if (BUDGET && c == ~0ull) {
+                    c = 0;
+                    if (lane == 0) s_expired = 1;
+                }
             } else {
                 uint32_t *A = staged && tri_words(W) <= room_words - r.p ? room + r.p : slab;
                 const Tri t{A};
-                if (staged) build_rows(g, b, (const uint32_t *)room, r.p, t, wib, nw);
-                else build_rows(g, b, a.ci + r.ids, r.p, t, wib, nw);
+                const bool built = staged ? build_rows<BUDGET>(a, g, b, (const uint32_t *)room, r.p, t, wib, nw)
+                                          : build_rows<BUDGET>(a, g, b, a.ci + r.ids, r.p, t, wib, nw);
+                if (BUDGET && !built && lane == 0) s_expired = 1;  // (the loop below ends at its first check, for all warps)
                 __syncthreads();
                 for (;;) {
                     uint32_t x = 0;
@@ -601,22 +622,22 @@ __device__ __forceinline__ uint64_t cta_list(const CliqueArgs &a, const Csr &g, 
     return sum;       // thread 0's
 }
 
-template <int K, bool ORDER>
+template <int K, bool ORDER, bool BUDGET>
 __global__ void __launch_bounds__(256, K == 5 ? 4 : 5) clique_kernel(const __grid_constant__ CliqueArgs a) {
     extern __shared__ uint32_t smem[];
     const uint32_t lane = lane_id(), wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const Csr g{a.rp, a.ci, a.fo, a.core.bits};
     uint64_t total = 0;
     const bool many = many_sparse(a);
-    if (!ORDER) total = cta_list<K>(a, g, smem, many);
+    if (!ORDER) total = cta_list<K, BUDGET>(a, g, smem, many);
     uint32_t *area = smem + wib * warp_area(K, ORDER, a.q_words);
     uint32_t *slab = a.scratch + ((uint64_t)blockIdx.x * nw + wib) * a.words_per_warp;
     uint64_t mine = 0;
     if (ORDER) {
-        warp_list<K, true>(a, g, 0, a.chunk, area, slab, many, mine);
+        warp_list<K, true, BUDGET>(a, g, 0, a.chunk, area, slab, many, mine);
     } else {
-        warp_list<K, false>(a, g, 1, 1u, area, slab, many, mine);
-        warp_list<K, false>(a, g, 2, 8u, area, slab, many, mine);
+        warp_list<K, false, BUDGET>(a, g, 1, 1u, area, slab, many, mine);
+        warp_list<K, false, BUDGET>(a, g, 2, 8u, area, slab, many, mine);
     }
     if (lane == 0) total += mine;
     if (lane == 0 && total) atomicAdd(a.out, (unsigned long long)total);
@@ -801,9 +822,9 @@ uint32_t clique_p_fit(uint32_t k, bool in_order, uint64_t words_per_warp, int wa
 
 template <int K, bool O>
 static int clique_occ(int wpb, size_t sm) {
-    cudaFuncSetAttribute(clique_kernel<K, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+    cudaFuncSetAttribute(clique_kernel<K, O, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, clique_kernel<K, O>, 32 * wpb, sm) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, clique_kernel<K, O, false>, 32 * wpb, sm) != cudaSuccess) return 0;
     return nb;
 }
 
@@ -831,16 +852,28 @@ cudaError_t clique_prepare_launch(const CliqueArgs &a, uint32_t k, int sms, cuda
     return cudaGetLastError();
 }
 
-cudaError_t clique_preload() {
+cudaError_t clique_preload(uint32_t k, bool in_order) {
     cudaFuncAttributes fa;
-    return cudaFuncGetAttributes(&fa, clique_prepare_kernel);
+    const cudaError_t e = cudaFuncGetAttributes(&fa, clique_prepare_kernel);
+    if (e != cudaSuccess) return e;
+    switch (k) {
+        case 3: return in_order ? cudaFuncGetAttributes(&fa, clique_kernel<3, true, true>) : cudaFuncGetAttributes(&fa, clique_kernel<3, false, true>);
+        case 4: return in_order ? cudaFuncGetAttributes(&fa, clique_kernel<4, true, true>) : cudaFuncGetAttributes(&fa, clique_kernel<4, false, true>);
+        case 5: return in_order ? cudaFuncGetAttributes(&fa, clique_kernel<5, true, true>) : cudaFuncGetAttributes(&fa, clique_kernel<5, false, true>);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+template <int K, bool O, bool B>
+static void clique_go_budget(const CliqueArgs &a, int blocks, int wpb, cudaStream_t st) {
+    cudaFuncSetAttribute(clique_kernel<K, O, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+    clique_kernel<K, O, B><<<blocks, 32 * wpb, 4ull * a.smem_words, st>>>(a);
 }
 
 template <int K, bool O>
 static void clique_go(const CliqueArgs &a, int blocks, int wpb, cudaStream_t st) {
-    const size_t sm = 4ull * a.smem_words;
-    cudaFuncSetAttribute(clique_kernel<K, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
-    clique_kernel<K, O><<<blocks, 32 * wpb, sm, st>>>(a);
+    if (a.deadline) clique_go_budget<K, O, true>(a, blocks, wpb, st);
+    else clique_go_budget<K, O, false>(a, blocks, wpb, st);
 }
 
 cudaError_t clique_launch(const CliqueArgs &a, uint32_t k, int blocks, int wpb, cudaStream_t st) {

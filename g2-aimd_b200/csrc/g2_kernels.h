@@ -106,7 +106,7 @@ int match_blocks_per_sm(int wpl, int warps_per_block, bool metrics, int ctas_per
 // Load the code of a budgeted launch (kernels load on their first use, which takes
 // milliseconds that would count against the budget).
 cudaError_t mce_preload(int wpl);
-cudaError_t clique_preload();  // the preparation kernel; clique_blocks_per_sm loads the other
+cudaError_t clique_preload(uint32_t k, bool in_order);
 cudaError_t mce_launch(int wpl, const MceArgs &a, int blocks, int warps_per_block, cudaStream_t st);
 // Advance a run's hand-off epoch in stream order (skipping 0, the value of a
 // never-published ready word), so runs captured in a CUDA graph stay distinct

@@ -889,6 +889,8 @@ __global__ void __launch_bounds__(256, MINB) match_kernel(MatchArgs a, int cliqu
                                                           const __grid_constant__ DevPlan pl) {
     extern __shared__ uint32_t smem[];
     __shared__ QueueWatch watch;
+    // (the rest list of a clique run is mostly empty)
+    if (a.spill_cycles == 0 && a.ntasks_dev && *a.ntasks_dev == 0) return;
     watch_init(&watch);
     __syncthreads();
     const uint32_t wib = threadIdx.x >> 5;

@@ -938,7 +938,7 @@ int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned lo
         q.deadline = a.deadline;
     }
     if (deadline_ms) {  // the budget starts on the device: the kernels' code has been loaded before it does
-        cudaError_t ed = rows ? g2::clique_preload() : cudaSuccess;
+        cudaError_t ed = rows ? g2::clique_preload(ctx->plan.k, cg.in_order) : cudaSuccess;
         if (ed == cudaSuccess) ed = g2::deadline_set(ctx->d_deadline, 1000000ull * deadline_ms, st);
         if (ed != cudaSuccess) return fail_cuda(ctx, ed, "deadline_set");
         ctx->launches++;

@@ -108,3 +108,40 @@ def test_budgeted_run_takes_roots_in_exact_cost_order(g2):
     done = rn[order] > 0
     k = int(done.sum())
     assert 20 < k < g.n and done[:k].all()
+
+
+@pytest.mark.parametrize("schedule", ["given", "heuristic"])
+@pytest.mark.parametrize("q,n,keep", [(0, 8000, 1.0), (24, 2500, 1.0), (25, 1100, 0.7)])
+def test_clique_budget_runs_out_inside_a_root(g2, q, n, keep, schedule):
+    """Counting the cliques over one root of n - 1 vertices takes many times the budget of
+    1 ms: the run ends soon after it, drops the root and says so; the finished roots of
+    a full run afterwards are unharmed."""
+    import time
+    from g2aimd.context import Context, Plan
+    plan = Plan.preset(q)
+    rng = np.random.default_rng(3)
+    a, b = np.triu_indices(n - 1, 1)
+    on = rng.random(a.size) < keep * (0.25 if n > 2000 else 1.0)
+    row = np.concatenate([np.zeros(n - 1, np.int64), a[on] + 1])
+    col = np.concatenate([np.arange(1, n), b[on] + 1])
+    key = np.sort(np.concatenate([row * n + col, col * n + row]))
+    rp = np.zeros(n + 1, np.uint64)
+    rp[1:] = np.cumsum(np.bincount(key // n, minlength=n))
+    g = g2.Graph(rp, (key % n).astype(np.uint32))
+    src = np.zeros(1, np.uint32)
+    with Context(0) as c:
+        c.load(g)
+        full = c.match(plan, sources=src, schedule=schedule)
+        t0 = time.perf_counter()
+        assert c.match(plan, sources=src, schedule=schedule) == full
+        full_ms = 1e3 * (time.perf_counter() - t0)
+        cost = np.zeros(1, np.uint64)
+        got = c.match(plan, sources=src, schedule=schedule, deadline_ms=1, root_cost=cost)  # loads the kernels
+        t0 = time.perf_counter()
+        got = c.match(plan, sources=src, schedule=schedule, deadline_ms=1, root_cost=cost)
+        ms = 1e3 * (time.perf_counter() - t0)
+        assert full_ms > 6, full_ms
+        assert c.expired and got == 0 and cost[0] == 0, (full_ms, ms)
+        # (5-cliques look at the clock once per highest vertex of the root)
+        assert ms < (0.9 if q == 25 else 0.5) * full_ms, (full_ms, ms)
+        assert c.match(plan, sources=src, schedule=schedule, deadline_ms=600000) == full and not c.expired
