@@ -36,6 +36,18 @@ int fail_cuda(g2_ctx *c, cudaError_t e, const char *where) {
     return e == cudaErrorMemoryAllocation ? G2_ERR_OOM : G2_ERR_CUDA;
 }
 
+// Memory of a view slot: the core's bit rows, which a run can do without, give way.
+cudaError_t malloc_slot(g2_ctx *c, void **p, uint64_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || !c->d_core_bits) return e;
+    cudaGetLastError();
+    cudaFree(c->d_core_bits);  // waits for the run that reads them
+    c->d_core_bits = nullptr;
+    c->core_bits_cap = 0;
+    c->last_mce.core.bits = nullptr;  // (its spill pass takes the general walk)
+    return cudaMalloc(p, bytes);
+}
+
 int fail_cuda_if(g2_ctx *c, cudaError_t e, const char *where) { return e == cudaSuccess ? G2_OK : fail_cuda(c, e, where); }
 
 }  // namespace g2rt
@@ -503,8 +515,16 @@ int gather_root_outputs(g2_ctx *ctx, const uint32_t *sources, uint64_t nsrc, uin
 // 16 6.2 / 0.33 (an earlier build of the kernels).
 uint64_t core_budget(uint64_t m) { return std::min<uint64_t>(std::max<uint64_t>(4 * m, 1u << 20), 2ull << 30); }
 
-// Geometry of the loaded graph's core bit rows; words = the matrix's size.
-g2::CoreBits core_geometry(const g2_ctx *ctx, uint64_t *words) {
+// A run over few roots gets a smaller matrix, 8 KB per root (2.7 ns of writing at
+// 3 TB/s, where a root of R-MAT s20 takes 3.9): with all of it ten roots of a graph of
+// 10^9 entries would write 2 GiB first.
+uint64_t run_budget(uint64_t m, uint64_t roots) {
+    return std::min<uint64_t>(core_budget(m), std::max<uint64_t>(roots * 8192, 1u << 20));
+}
+
+// Geometry of the loaded graph's core bit rows for a run over `roots`; words = the
+// matrix's size.
+g2::CoreBits core_geometry(const g2_ctx *ctx, uint64_t roots, uint64_t *words) {
     g2::CoreBits cb{};
     if (ctx->batch_off.size() > 2) {
         cb.blocks = ctx->d_core_blocks;
@@ -513,7 +533,7 @@ g2::CoreBits core_geometry(const g2_ctx *ctx, uint64_t *words) {
         *words = ctx->core_words;
     } else {
         cb.nblocks = 1;
-        cb.one = g2::core_block_of(0, (uint32_t)ctx->n, core_budget(ctx->m), 0, 0);
+        cb.one = g2::core_block_of(0, (uint32_t)ctx->n, run_budget(ctx->m, roots), 0, 0);
         cb.rows = cb.one.end - cb.one.base;
         *words = (uint64_t)cb.rows * cb.one.stride;
     }
@@ -522,12 +542,13 @@ g2::CoreBits core_geometry(const g2_ctx *ctx, uint64_t *words) {
 
 constexpr uint64_t kCliquePieces = 1u << 16;  // list entries for pieces of heavy roots
 
-// The core matrix and the task lists of clique runs over up to `tasks` tasks (0: the matrix alone):
+// The core matrix of a run over `roots`, and the task lists of clique runs over up to
+// `tasks` tasks (0: the matrix alone):
 // G2_OK, or G2_ERR_OOM where the run has to do without them (no memory left, or
 // a stream capture, in which nothing is allocated).
-int ensure_clique(g2_ctx *ctx, uint64_t tasks, cudaStream_t st, g2::CoreBits *cb) {
+int ensure_clique(g2_ctx *ctx, uint64_t roots, uint64_t tasks, cudaStream_t st, g2::CoreBits *cb) {
     uint64_t words = 0;
-    *cb = core_geometry(ctx, &words);
+    *cb = core_geometry(ctx, roots, &words);
     words = std::max<uint64_t>(words, 4);
     if (tasks) tasks = 5 * (tasks + kCliquePieces);  // four lists and the pieces
     if (ctx->core_bits_cap < words || ctx->clists_cap < tasks) {
@@ -535,6 +556,8 @@ int ensure_clique(g2_ctx *ctx, uint64_t tasks, cudaStream_t st, g2::CoreBits *cb
         G2_TRY(cudaStreamIsCapturing(st, &cs));
         if (cs != cudaStreamCaptureStatusNone) return G2_ERR_OOM;
     }
+    // (by half at least, as the view slots grow: the views of a run differ in size)
+    if (words > ctx->core_bits_cap) words = std::max(words, std::min<uint64_t>(ctx->core_bits_cap * 3 / 2, 512u << 20));
     int rc = grow(ctx, ctx->d_core_bits, ctx->core_bits_cap, words, "core bit rows");
     if (!rc && tasks) rc = grow(ctx, ctx->d_clists, ctx->clists_cap, tasks, "clique task lists");
     if (rc == G2_ERR_OOM) cudaGetLastError();
@@ -660,7 +683,7 @@ int mce_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned long
     if (const char *e = getenv("G2_HIST_FOLD"))  // (tests cross it with few nodes)
         base.hist_fold = 1u << std::min<uint32_t>((uint32_t)strtoul(e, nullptr, 10), 24u);
     if (!base.work && !deadline_ms && !tl.split) {  // (those runs take the general walk)
-        rc = ensure_clique(ctx, 0, st, &base.core);
+        rc = ensure_clique(ctx, tl.cap, 0, st, &base.core);
         if (rc && rc != G2_ERR_OOM) return rc;
         if (rc) base.core.bits = nullptr;
     }
@@ -901,7 +924,7 @@ int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned lo
     CliqueGrid cg{};
     bool rows = clique_run(ctx, o);
     if (rows) {
-        rc = ensure_clique(ctx, std::max<uint64_t>(tl.cap, 1), st, &q.core);
+        rc = ensure_clique(ctx, tl.cap, std::max<uint64_t>(tl.cap, 1), st, &q.core);
         if (rc && rc != G2_ERR_OOM) return rc;
         rows = rc == G2_OK;
     }
@@ -1067,7 +1090,7 @@ int g2_reserve(g2_ctx *ctx, uint64_t max_sources) {
         if (!rc && !ctx->d_ntask) rc = grow(ctx, ctx->d_ntask, ctx->ntask_cap, 1, "task count");
         if (rc) return rc;
         g2::CoreBits cb;
-        rc = ensure_clique(ctx, ctx->tasks_cap, nullptr, &cb);
+        rc = ensure_clique(ctx, ctx->tasks_cap, ctx->tasks_cap, nullptr, &cb);
         if (rc && rc != G2_ERR_OOM) return rc;
         size_t sort_need = 0, scan_need = 0;
         cub::DeviceRadixSort::SortKeys(nullptr, sort_need, ctx->d_keys, ctx->d_keys2, (int)cap, 0, 64);

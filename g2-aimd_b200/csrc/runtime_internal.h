@@ -116,6 +116,9 @@ int g2_after_load(g2_ctx *ctx);
 void view_builder_free(void *builder);
 int fail_cuda_if(g2_ctx *c, cudaError_t e, const char *where);
 
+// cudaMalloc of a view slot (frees the core's bit rows if that makes it fit).
+cudaError_t malloc_slot(g2_ctx *c, void **p, uint64_t bytes);
+
 #define G2_TRY(call)                                             \
     do {                                                         \
         cudaError_t _e = (call);                                 \

@@ -440,7 +440,7 @@ int DeviceViewBuilder::build(const uint32_t *roots, uint64_t nroots, void **buf,
         if (*buf) cudaFree(*buf);  // synchronises: the slot's last run has ended anyway
         *buf = nullptr;
         *cap = 0;
-        G2_TRY(cudaMalloc(buf, want));
+        G2_TRY(malloc_slot(ctx, buf, want));
         *cap = want;
     }
     char *b = static_cast<char *>(*buf);

@@ -216,7 +216,7 @@ struct ViewDevice {
             if (buf[d]) cudaFree(buf[d]);  // synchronises: the slot's last run has ended anyway
             buf[d] = nullptr;
             cap[d] = 0;
-            G2_TRY(cudaMalloc(&buf[d], want));
+            G2_TRY(malloc_slot(ctx, &buf[d], want));
             cap[d] = want;
         }
         G2_TRY(cudaStreamWaitEvent(copy, done[d], 0));

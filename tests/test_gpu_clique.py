@@ -54,10 +54,58 @@ def test_ids_without_bit_rows(g2, orc, ctx, q):
         assert ctx.match(plan, sources=src, **kw) == int(want["root_counts"][src].sum())
 
 
+@pytest.mark.parametrize("take", [1, 7, 300])
+def test_few_roots_get_a_small_matrix(g2, orc, ctx, take):
+    """A run's bit rows are sized by its roots (8 KB each, 1 MB at least): of these
+    70,000 vertices 2,900, 2,900 and 4,400 get one, all runs after one with all."""
+    from g2aimd.context import Plan
+    g = g2.Graph.rmat(16, 16, seed=3).degeneracy_recoded()
+    rng = np.random.default_rng(take)
+    fwd = np.array([int(r) for r in g.degrees()])
+    src = rng.choice(np.flatnonzero(fwd > 40), take, replace=False).astype(np.uint32)
+    ctx.load(g)
+    for q in (0, 24):
+        plan = Plan.preset(q)
+        want = orc.match(g, plan, roots=src, threads=8)["count"]
+        for kw in ({}, {"schedule": "heuristic"}):
+            assert ctx.match(plan, **kw) > 0
+            assert ctx.match(plan, sources=src, **kw) == want, (q, kw)
+    want = orc.mce(g, roots=src, threads=8)
+    c, h = ctx.mce(sources=src)
+    assert c == want["count"] and np.array_equal(h, want["hist"][:h.size])
+
+
+@pytest.mark.parametrize("words", [0, 64 * 37])
+def test_wide_5_clique_roots(g2, orc, words):
+    """A root of 640 vertices one of which is adjacent to 420 earlier ones (more than are
+    compressed into rows of their own), beside roots up to 130 wide: rows in shared
+    memory, in slabs and, with small scratch, beyond them."""
+    from g2aimd.context import Context, Plan
+    plan = Plan.preset(25)
+    rng = np.random.default_rng(12)
+    n = 641
+    e = [np.stack([np.zeros(640, int), np.arange(1, n)], 1)]
+    a, b = np.triu_indices(520, 1)
+    on = rng.random(a.size) < 0.06
+    e.append(np.stack([a[on] + 1, b[on] + 1], 1))
+    e.append(np.stack([rng.choice(np.arange(1, 521), 420, replace=False), np.full(420, 600)], 1))
+    g = _csr(g2, n, np.concatenate(e))
+    fwd = g.neighbors(0)
+    assert fwd.size == 640 and int((g.neighbors(600) < 600).sum()) > 256
+    want = orc.match(g, plan, threads=8, per_root=True)
+    launch = dict(blocks=148, warps_per_block=8) if words else {}
+    with Context(0, scratch_bytes=148 * 8 * words * 4) as c:
+        c.load(g)
+        for kw in ({}, {"schedule": "heuristic"}, {"schedule": "heuristic", "split": True, "granularity": 256}):
+            rc = np.zeros(g.n, np.uint64)
+            assert c.match(plan, root_counts=rc, **dict(launch, **kw)) == want["count"] > 0, (words, kw)
+            assert np.array_equal(rc, want["root_counts"]), (words, kw)
+
+
 @pytest.mark.parametrize("q", [0, 24, 25])
 def test_rows_in_slabs_and_beyond(g2, orc, q):
-    """A complete-ish core of 420 vertices: its rows exceed the shared memory of a
-    CTA of one warp and, with small scratch, the slabs too (the rest list)."""
+    """Dense cores of 700 vertices (3- and 4-cliques: rows in shared memory and, with small
+    scratch, beyond the slabs, the rest list) and of 420 (5-cliques, up to 97 wide)."""
     from g2aimd.context import Context, Plan
     plan = Plan.preset(q)
     rng = np.random.default_rng(5)
