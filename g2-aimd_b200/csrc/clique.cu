@@ -325,6 +325,7 @@ __device__ __forceinline__ bool many_sparse(const CliqueArgs &a) { return a.by_c
 // A root to the rest list (one lane).
 __device__ __forceinline__ void to_rest(const CliqueArgs &a, uint32_t task) {
     a.lists[3 * a.list_cap + atomicAdd(a.counts + 3, 1ull)] = task;
+    atomicOr(a.status, kStatusRest);
 }
 
 // p <= 32: lane j holds P0[j] and its row.  Warp total.
@@ -771,7 +772,10 @@ __global__ void __launch_bounds__(256) clique_prepare_kernel(const __grid_consta
                 if (lane >= (uint32_t)o) incl += y;
             }
             unsigned long long at = 0;
-            if (lane == 31) at = atomicAdd(a.counts + l, (unsigned long long)incl);
+            if (lane == 31) {
+                at = atomicAdd(a.counts + l, (unsigned long long)incl);
+                if (l == 3) atomicOr(a.status, kStatusRest);
+            }
             at = __shfl_sync(G2_FULL, at, 31);
             if (list != l) continue;
             at += incl - copies;

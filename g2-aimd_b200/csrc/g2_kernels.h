@@ -19,6 +19,8 @@ constexpr int kStatusBadPlan = 8;        // plan arrays inconsistent
 constexpr int kStatusWaitLimit = 16;     // a bounded device wait ran out
 constexpr int kStatusDeadline = 32;      // the run's time budget ran out (MCE)
 
+constexpr int kStatusRest = 64;          // (no error) a clique run's rest list has entries
+
 // An MCE pass entry with this bit set is a spilled record id, else a task id.
 constexpr uint32_t kRecordBit = 0x80000000u;
 // Depth word of a record slot whose reservation ran past the buffer's end.

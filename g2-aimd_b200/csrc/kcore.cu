@@ -304,8 +304,9 @@ __global__ void recode_scatter_kernel(const uint64_t *rp, const uint32_t *ci, co
 // that names a neighbour twice (not a deduplicated list) yields fewer ids than it
 // has entries: *repeated is set and the caller sorts all rows instead.  CUB's
 // segmented sort gives such a row to one CTA for four radix passes over global
-// memory (R-MAT s18: 978 us, and 756 us to scatter the rows a warp each; rows of
-// 1024 entries on here: 85 + 135 us, with 846 us left in the segmented sort).
+// memory (R-MAT s18: 978 us, and 756 us to scatter the rows a warp each; measured
+// with rows of 1024 entries on here: 85 + 135 us, and 846 us left in the segmented
+// sort; the line stands at n / 1024 entries, 256 there).
 constexpr uint32_t kSpanWords = 32768, kSpan = 32u * kSpanWords;  // 128 KB of shared memory
 // rows from here on: a row costs a look at n / 32 words, so longer rows for more vertices
 inline uint64_t big_row(uint64_t n) { return n >> 10 > 256 ? n >> 10 : 256; }

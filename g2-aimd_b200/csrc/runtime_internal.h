@@ -83,6 +83,11 @@ struct g2_ctx {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // around the enumeration passes
     g2::MceArgs last_mce{};            // arguments of the last MCE enqueue (host-spill pass)
     int last_mce_wpl = 1;
+    struct {                           // the rest list's launch, where a synchronous clique run puts it off
+        g2::MatchArgs a{};
+        int blocks = 0, wpb = 0, wpl = 0, ctas = 0;
+        bool pending = false;
+    } rest;
     uint64_t host_spill_bytes = 1ull << 30;  // managed slab for roots no device slab holds
     void *h_spill = nullptr;
     uint64_t h_spill_bytes = 0;
@@ -149,8 +154,10 @@ int prepare_tasks(g2_ctx *ctx, const uint32_t *sources, uint64_t nsrc, bool on_d
 // The enumeration passes of one run, enqueued on `st`.
 int mce_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned long long *d_out, uint32_t hist_len,
                 uint64_t *d_root_nodes, uint64_t *d_root_cost, cudaStream_t st, uint64_t *d_root_cliques = nullptr);
+// rest_later: a clique run's rest list is left to match_rest, which the caller calls
+// if the status word has kStatusRest.
 int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned long long *d_out,
-                  uint64_t *d_root_nodes, uint64_t *d_root_cost, cudaStream_t st);
+                  uint64_t *d_root_nodes, uint64_t *d_root_cost, cudaStream_t st, bool rest_later = false);
 // After a synchronous MCE run: roots no device slab held, on the managed spill slab.
 int mce_host_spill(g2_ctx *ctx, cudaStream_t st);
 // Device-stream MCE runs: the same pass in stream order, then a flag for entries left.
