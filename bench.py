@@ -604,6 +604,18 @@ def c4_leg(Context, CostModel, Plan, models, local, seed, torch, stream, budget_
     return out
 
 
+def clique_pass_bytes(n, m):
+    """Bytes of one clique pass over every root: row pointers, columns and forward
+    offsets read once, the bit rows of the core (K ids, a multiple of 128 with K^2 / 8
+    up to the columns' bytes, 1 MB to 2 GiB; csrc/runtime.cu core_budget) written and
+    read once, one task id per root."""
+    budget, k = min(max(4 * m, 1 << 20), 2 << 30), 0
+    while k < n and (k + 128) ** 2 // 8 <= budget:
+        k += 128
+    k = min(k, n)
+    return 8 * (n + 1) + 4 * m + 4 * n + 2 * 4 * k * ((k + 127) // 128 * 4) + 4 * n + 8
+
+
 def headline_profile():
     """Figures of the headline kernel's ncu capture committed under profiles/
     (R-MAT s20 ef16 seed 1, 4-cliques): DRAM bytes per launch and warp
@@ -1031,8 +1043,10 @@ def run_ours(a):
                              f"degeneracy order, heaviest first), {cs['seconds']:.1f} s, plan-driven enumeration "
                              "with the reference planner's plan (oracle/g2_oracle.c, all host threads)"}
     peak, peak_kind = measured_peak()
-    stream_bytes = g.clique_stream_bytes(4)
-    achieved = stream_bytes / (kern_ms / 1000.0) / 1e9 if kern_ms else None
+    # what the pass cannot do without: the CSR and forward offsets once, the core's bit
+    # rows written and read once, the task list and the count
+    alg_bytes = clique_pass_bytes(g.n, g.m)
+    achieved = alg_bytes / (kern_ms / 1000.0) / 1e9 if kern_ms else None
     prof = headline_profile() if (a.scale, a.edge_factor, a.seed) == (20, 16, 1) else {}
     csum = clk.summary()
     issue = None
@@ -1054,10 +1068,11 @@ def run_ours(a):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None,
                          "traffic": prof.get("traffic"),
-                         "kernel": "clique_prepare_kernel + clique_kernel<4,0> (core bit rows), main pass", "kernel_ms": kern_ms,
-                         "algorithmic_bytes": stream_bytes, "peak_kind": peak_kind,
+                         "kernel": "clique_prepare_kernel + clique_kernel<4,0,0> (core bit rows), main pass",
+                         "kernel_ms": kern_ms, "algorithmic_bytes": alg_bytes, "peak_kind": peak_kind,
                          "binding": "instruction issue (see issue.frac); the HBM fraction is far from binding",
                          "issue": issue,
+                         "list_scan_model_bytes": g.clique_stream_bytes(4),
                          "merge_model_bytes": work_bytes,
                          "merge_model_gbs": work_bytes / (kern_ms / 1000.0) / 1e9 if kern_ms else None},
             "clocks": csum, "gpu_launches": int(launches_per_step * a.steps),

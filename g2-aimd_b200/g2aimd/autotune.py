@@ -6,6 +6,9 @@ results never depend on:
   * split granularity   heavy-root tasks aim at total / (g x warps) cost
   * warps per CTA       4 or 8 (the persistent grid keeps 32 warps per SM)
   * queue chunk         tasks taken per atomic on the device queue
+    (none of the three, nor the register budget, acts on 3- to 5-clique runs in
+    schedule order, which share roots among CTAs of 8 warps: there a sweep times
+    the same launch again)
   * intersection path   clique plans: bitmap (0) or generic plan interpreter (1)
   * register budget     GMatch kernel built for 4 or 6 CTAs of 256 threads per SM
   * MCE hand-off        check interval of walks for idle warps (bench's MCE space)

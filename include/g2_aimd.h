@@ -102,7 +102,8 @@ typedef struct g2_plan {
                                  set with g2_set_model (features + MLP fused into
                                  task generation); plan walks split heavy roots by
                                  default (3- to 5-clique runs share them among a
-                                 CTA's warps instead)                             */
+                                 CTA's warps instead, unless some root has more than
+                                 2,048 forward neighbours)                        */
 
 /*
  * Run options.  Zero-initialise and set what you need; 0 means "default".
@@ -127,7 +128,8 @@ typedef struct g2_opts {
     uint64_t *root_cost;        /* optional host out: SM cycles per source (summed
                                    over its split tasks)                            */
     uint32_t chunk;             /* tasks taken per queue atomic (0 = 1, MCE more among
-                                   its light tasks; 4 for plan walks)               */
+                                   its light tasks while every warp has enough of
+                                   them left; 4 for plan walks)                     */
     uint32_t spill_kcycles;     /* MCE and plan walks of non-clique plans: every this
                                    many thousand SM cycles a walk checks for idle
                                    warps and hands them the pending work of its
@@ -290,7 +292,9 @@ int g2_last_work_bytes(g2_ctx *ctx, uint64_t *bytes);
 
 /* Degeneracy order of the loaded graph computed on the device (replaces the
  * host peeling of kmeans/kcore.cpp:39-191): perm[v] = new id of v, core[v] =
- * core number (optional).  Equal to g2_degeneracy_order's output. */
+ * core number (optional).  Equal to g2_degeneracy_order's output.
+ * G2_ERR_TIMEOUT: a wait of the kernel's grid barrier ran out (2^37 SM cycles; the
+ * environment variable G2_PEEL_WAIT sets another limit, G2_PEEL_BLOCKS fewer CTAs). */
 int g2_degeneracy_order_device(g2_ctx *ctx, uint32_t *perm, uint32_t *core);
 
 /*
