@@ -700,6 +700,27 @@ __global__ void __launch_bounds__(256) core_rows_kernel(const __grid_constant__ 
               ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, ((uint64_t)gridDim.x * blockDim.x) >> 5);
 }
 
+// Roots of a loaded graph that may leave the tiles (4 heads each; a very wide one
+// counts as 1024).
+__global__ void __launch_bounds__(256) sparse_roots_kernel(const __grid_constant__ CliqueArgs a, uint64_t n,
+                                                           unsigned int *count) {
+    unsigned int c = 0;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t ids = ldg(a.rp + v) + ldg(a.fo + v), p = ldg(a.rp + v + 1) - ids;
+        if (p <= kFewHeads) continue;
+        if (p <= kSparseP) {
+            c += small_leaves_tiles(a, a.core.one, ids, p);
+            continue;
+        }
+        uint64_t sum = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++) sum += forward_length(a, ldg(a.ci + ids + p * (2 * i + 1) / 8u));
+        if (sum / 4u * 16u < p || (sum / 4u + 32u < 3u * p && heads_far(a, a.core.one, ids, p))) c += p > kWideP ? 1024u : 1u;
+    }
+    c = __reduce_add_sync(G2_FULL, c);
+    if (lane_id() == 0 && c) atomicAdd(count, c < (1u << 20) ? c : 1u << 20);
+}
+
 // The task lists and the core's bit rows.
 __global__ void __launch_bounds__(256) clique_prepare_kernel(const __grid_constant__ CliqueArgs a, uint32_t k) {
     __shared__ __align__(16) uint32_t seg_all[8][kSeg];
@@ -846,6 +867,14 @@ cudaError_t core_rows_launch(const CoreBits &core, uint32_t *bits, const uint64_
                              const uint32_t *fo, int sms, cudaStream_t st) {
     const uint64_t blocks = ((uint64_t)core.rows + 7) / 8, cap = 8ull * (uint64_t)sms;
     if (blocks) core_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(core, rp, ci, fo, bits);
+    return cudaGetLastError();
+}
+
+cudaError_t sparse_roots_launch(const uint64_t *rp, const uint32_t *ci, const uint32_t *fo, uint64_t n,
+                                const CoreBlock &core, int sms, unsigned int *count) {
+    CliqueArgs a{};
+    a.rp = rp, a.ci = ci, a.fo = fo, a.core.one = core;
+    sparse_roots_kernel<<<8 * sms, 256>>>(a, n, count);
     return cudaGetLastError();
 }
 

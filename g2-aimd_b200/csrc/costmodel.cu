@@ -396,8 +396,13 @@ __global__ void __launch_bounds__(128) score_kernel(const uint32_t *src, uint64_
         const float *f = X + row * F + 2 * q;
         return make_float2((f[0] - m0) * s0, (f[1] - m1) * s1);
     };
+    // rows two steps ahead and their features one step ahead of the arithmetic
+    uint64_t r0 = row_of(warp * 16 + g), r1 = row_of(warp * 16 + g + 8);
+    float2 x0 = load(r0), x1 = load(r1);
+    r0 = row_of((warp + nwarps) * 16 + g), r1 = row_of((warp + nwarps) * 16 + g + 8);
     for (uint64_t base = warp * 16; base < n; base += nwarps * 16) {
-        const float2 x0 = load(row_of(base + g)), x1 = load(row_of(base + g + 8));
+        const float2 y0n = load(r0), y1n = load(r1);
+        r0 = row_of(base + 2 * nwarps * 16 + g), r1 = row_of(base + 2 * nwarps * 16 + g + 8);
         const uint32_t ax[4] = {pack_bf16(x0.x, x0.y), pack_bf16(x1.x, x1.y), 0u, 0u};
         uint32_t h[H / 16][4];
 #pragma unroll
@@ -434,6 +439,8 @@ __global__ void __launch_bounds__(128) score_kernel(const uint32_t *src, uint64_
                 local += cc;
             }
         }
+        x0 = y0n;
+        x1 = y1n;
     }
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(G2_FULL, local, o);
     if (lane == 0 && total && local != 0.f) atomicAdd(total, local);

@@ -232,6 +232,10 @@ int clique_blocks_per_sm(uint32_t k, bool in_order, int warps_per_block, uint32_
 // The core's bit rows alone (core.bits), in stream order.
 cudaError_t core_rows_launch(const CoreBits &core, uint32_t *bits, const uint64_t *rp, const uint32_t *ci,
                              const uint32_t *fo, int sms, cudaStream_t st);
+// *count += roots of a graph that may be cheaper by their forward lists than by tiles
+// over the block `core` (legacy stream).
+cudaError_t sparse_roots_launch(const uint64_t *rp, const uint32_t *ci, const uint32_t *fo, uint64_t n,
+                                const CoreBlock &core, int sms, unsigned int *count);
 cudaError_t clique_prepare_launch(const CliqueArgs &a, uint32_t k, int sms, cudaStream_t st);
 cudaError_t clique_launch(const CliqueArgs &a, uint32_t k, int blocks, int warps_per_block, cudaStream_t st);
 

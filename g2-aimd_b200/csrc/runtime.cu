@@ -954,7 +954,12 @@ int match_enqueue(g2_ctx *ctx, const TaskList &tl, const g2_opts *o, unsigned lo
         q.q_words = cg.q_words;
         q.cta_min = g2::clique_cta_min(ctx->plan.k);
         q.p_fit = g2::clique_p_fit(ctx->plan.k, cg.in_order, q.words_per_warp, cg.wpb);
-        q.by_cost = g2::clique_by_cost(ctx->max_fwd, q.core.rows == ctx->n);
+        // (a graph with hardly a sparse root keeps the tiles for all: an empty launch for
+        // the rest list costs 36 us between others; few roots have a smaller matrix than
+        // the one looked at when the graph was loaded)
+        q.by_cost = g2::clique_by_cost(ctx->max_fwd, q.core.rows == ctx->n) &&
+                    !(ctx->dense_roots && ctx->batch_off.size() <= 2 &&
+                      run_budget(ctx->m, tl.cap) == core_budget(ctx->m));
         q.out = d_out;
         q.root_nodes = d_root_nodes;
         q.root_cost = d_root_cost;
@@ -1266,15 +1271,21 @@ static int after_load(g2_ctx *ctx) {
     ctx->batch_off.clear();  // a batch load sets it again afterwards
     ctx->feat_valid = false;
     ctx->core_loaded = false;  // core numbers belong to the previous graph (buffer kept)
-    if (!ctx->d_fwdmax) G2_TRY(cudaMalloc(&ctx->d_fwdmax, sizeof(unsigned int)));
+    if (!ctx->d_fwdmax) G2_TRY(cudaMalloc(&ctx->d_fwdmax, 2 * sizeof(unsigned int)));
     unsigned int *d_max = ctx->d_fwdmax;
-    G2_TRY(cudaMemset(d_max, 0, sizeof(unsigned int)));
-    if (ctx->n) forward_offsets_kernel<<<ctx->sm_count * 4, 256>>>(ctx->d_rp, ctx->d_ci, ctx->n, ctx->d_fo, d_max);
-    ctx->launches++;
-    unsigned int h = 0;
-    cudaError_t e = cudaMemcpy(&h, d_max, sizeof(unsigned int), cudaMemcpyDeviceToHost);
+    G2_TRY(cudaMemset(d_max, 0, 2 * sizeof(unsigned int)));
+    if (ctx->n) {
+        forward_offsets_kernel<<<ctx->sm_count * 4, 256>>>(ctx->d_rp, ctx->d_ci, ctx->n, ctx->d_fo, d_max);
+        const g2::CoreBlock core = g2::core_block_of(0, (uint32_t)ctx->n, core_budget(ctx->m), 0, 0);
+        cudaError_t es = g2::sparse_roots_launch(ctx->d_rp, ctx->d_ci, ctx->d_fo, ctx->n, core, ctx->sm_count, d_max + 1);
+        if (es != cudaSuccess) return fail_cuda(ctx, es, "sparse_roots_launch");
+    }
+    ctx->launches += 2;
+    unsigned int h[2] = {0, 0};
+    cudaError_t e = cudaMemcpy(h, d_max, sizeof(h), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return fail_cuda(ctx, e, "fwd_max");
-    ctx->max_fwd = h;
+    ctx->max_fwd = h[0];
+    ctx->dense_roots = h[1] < 64;
     return G2_OK;
 }
 

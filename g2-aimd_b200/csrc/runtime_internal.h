@@ -28,7 +28,8 @@ struct g2_ctx {
     uint32_t *d_core = nullptr;  // optional core numbers (cost-model feature)
     bool core_loaded = false;    // d_core holds the loaded graph's core numbers
     uint64_t rp_cap = 0, ci_cap = 0;       // owned CSR buffers (entries), reused by later loads
-    unsigned int *d_fwdmax = nullptr;      // max forward degree of a load
+    unsigned int *d_fwdmax = nullptr;      // max forward degree of a load, and its sparse roots
+    bool dense_roots = false;              // next to no root of the loaded graph leaves the tiles of a full run
     uint64_t core_cap = 0;
     // work buffers
     uint32_t *d_scratch = nullptr;

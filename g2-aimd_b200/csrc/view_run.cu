@@ -242,6 +242,7 @@ struct ViewDevice {
         ctx->batch_off.clear();
         ctx->feat_valid = false;
         ctx->core_loaded = false;
+        ctx->dense_roots = false;  // not looked at
         return reinterpret_cast<uint32_t *>(b + L.src);
     }
 
