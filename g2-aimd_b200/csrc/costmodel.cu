@@ -474,7 +474,7 @@ cudaError_t adam_launch(float *params, float *mom, float *vel, const float *grad
 
 cudaError_t score_launch(const uint32_t *src, uint64_t n, const float *X, const float *params, const float *norm,
                          float *pred, float *cost, float *total, int sms, cudaStream_t st) {
-    const uint64_t blocks = (n + 63) / 64, cap = 4ull * (uint64_t)sms;
+    const uint64_t blocks = (n + 63) / 64, cap = 3ull * (uint64_t)sms;  // what is resident at once
     score_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks < cap ? blocks : cap), 128, 0, st>>>(src, n, X, params, norm,
                                                                                          pred, cost, total);
     return cudaGetLastError();
